@@ -88,6 +88,12 @@ struct hc_ctx {
     double *phs, *rhs;           // colour-split potential and density (FP64 solve)
     double *plm;                 // MUSCL-Hancock face-state buffer (20 values per cell; recon = 1)
     float *e32, *r32, *e32b;     // mixed precision correction (ping-pong) / residual
+    // resident sweeps (sor_resident.cuh): the grid's blocks, the message rows
+    // and the number of the next launch's first sweep
+    int resident;                // 0 not looked at yet, 1 in use, -1 the grid does not fit
+    ResPlan rplan;
+    void *exch;
+    unsigned epoch;
     double *gx, *gy, *gz;
     double *res;
     int res_cap;
@@ -225,7 +231,7 @@ static void free_ctx(hc_ctx *c)
         }
     cudaFree(c->phi); cudaFree(c->phig); cudaFree(c->rho_ext); cudaFree(c->phi2);
     cudaFree(c->phs); cudaFree(c->rhs); cudaFree(c->plm); cudaFree(c->slab_buf);
-    cudaFree(c->e32); cudaFree(c->r32); cudaFree(c->e32b);
+    cudaFree(c->e32); cudaFree(c->r32); cudaFree(c->e32b); cudaFree(c->exch);
     cudaFree(c->gx); cudaFree(c->gy); cudaFree(c->gz);
     cudaFree(c->res); cudaFree(c->scratch); cudaFree(c->mom); cudaFree(c->cons_part);
     cudaFree(c->sc); cudaFree(c->stage);
@@ -579,6 +585,30 @@ static int next_batch(const double *slots, int nb, double thresh, int prev)
     return std::min(prev * 2, 256);
 }
 
+// Whether the default sweeps of this context run resident (words of `elem`
+// bytes, the same for every solve of a context but those of a host density
+// in an FP32 one, which sweep in FP64); allocates the message rows once.
+static bool resident_sweeps(hc_ctx *c, size_t elem)
+{
+    if (c->cfg.sor_depth != 0 || (elem == 8) != (c->cfg.precision == HC_FP64)) return false;
+    if (c->resident == 0) {
+        c->resident = -1;
+        if (grav_resident_plan(c->g, elem, &c->rplan)) {
+            void *p = nullptr;
+            if (cudaMalloc(&p, c->rplan.exch_bytes) != cudaSuccess) {
+                (void)cudaGetLastError();   // no room: the separate sweeps need none
+            } else if (cudaMemsetAsync(p, 0, c->rplan.exch_bytes, c->s) != cudaSuccess) {
+                cudaFree(p);
+            } else {
+                c->exch = p;
+                c->epoch = 1;
+                c->resident = 1;
+            }
+        }
+    }
+    return c->resident == 1;
+}
+
 // Red-black SOR to tolerance, FP64 (gravity_solve_potential,
 // gravity_solver_3d.c:510-747).  Returns 0 / -1 like the reference, or a
 // negative HC_ERR_* code.
@@ -603,6 +633,7 @@ static int sor_fp64(hc_ctx *c, const double *rho)
     // place between phi (buf 0) and phi2 (buf 1): iteration t reads buf[t%2],
     // writes buf[(t+1)%2].  All three give the same iterates.
     const bool split = c->cfg.sor_depth == 0 && c->g.nz >= 3;
+    const bool resident = split && resident_sweeps(c, sizeof(double));
     const bool wave = c->cfg.sor_depth >= 1 && c->g.nz >= 3;
     double *buf[2] = { c->phi, c->phi2 };
     if (split) {
@@ -659,16 +690,24 @@ static int sor_fp64(hc_ctx *c, const double *rho)
         c->launches += 1;
     }
     int it = 1, done = 0, last = 0;
-    int batch = 16;
+    // a resident launch stops by itself: no polls in between, the cap only
+    // bounds one launch's duration
+    int batch = resident ? 4096 : 16;
     while (true) {
         int end = std::min(a.max_iter, it + batch);
         {
             FamTimer t(c, FAM_SOR);
-            for (int q = it; q < end; q++) {
-                rc = one_iter(q);
-                if (rc) return rc;
+            if (resident && end > it) {
+                CK(grav_sor_resident(a, c->phs, c->rhs, c->rplan, c->exch, c->epoch, it, end - it, c->s));
+                c->epoch += 4u * (unsigned)(end - it) + 16u;
+                c->sor_launches += 1;
+            } else {
+                for (int q = it; q < end; q++) {
+                    rc = one_iter(q);
+                    if (rc) return rc;
+                }
+                CK(grav_check(a, end, c->s));
             }
-            CK(grav_check(a, end, c->s));
         }
         c->launches += 1;
         CK(cudaMemcpyAsync(&c->hsc->done, &c->sc->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->s));
@@ -682,7 +721,7 @@ static int sor_fp64(hc_ctx *c, const double *rho)
         last = c->hsc->last_iter;
         if (done || end >= a.max_iter) break;
         it = end;
-        batch = next_batch(c->hslots, nb, a.tol, batch);
+        if (!resident) batch = next_batch(c->hslots, nb, a.tol, batch);
     }
     int used = done ? last : a.max_iter;
     if (wave && (used & 1)) std::swap(c->phi, c->phi2);   // result in buf[used % 2]
@@ -719,6 +758,7 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
     // one in-place kernel per colour on the natural layout; >= 1: wavefront
     // passes of that many FP32 iterations per HBM pass on the natural layout
     const bool split = (c->cfg.sor_depth == 0 || c->cfg.sor_depth == -2 || c->cfg.sor_depth == -3) && c->g.nz >= 3;
+    const bool resident = split && resident_sweeps(c, sizeof(float));
     const bool wave2 = split && c->cfg.sor_depth == -2 && mixed_wave_split_ok(c->g);
     const int depth = wave2 ? 2 : (split ? -1 : c->cfg.sor_depth);
     int rc = ensure_res(c, a.max_iter);
@@ -840,7 +880,12 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
             int end = std::min(budget, it + batch);
             {
                 FamTimer t(c, FAM_SOR);
-                if (wave2) {
+                if (resident) {
+                    CK(mixed_sor32_resident(a, c->e32, c->r32, c->rplan, c->exch, c->epoch, it, end - it, thresh,
+                                            c->s));
+                    c->epoch += 4u * (unsigned)(end - it) + 16u;
+                    c->sor_launches += 1;
+                } else if (wave2) {
                     for (int q = it; q < end; q += 2) {
                         CK(mixed_sor32_split_pass(a, eb[(q / 2) & 1], eb[((q / 2) + 1) & 1], c->r32, q, thresh, c->s));
                         c->launches += 1;
@@ -872,7 +917,7 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
                     }
                     end = it + ((end - it + depth - 1) / depth) * depth;
                 }
-                CK(mixed_check(a, end, thresh, c->s));
+                if (!resident) CK(mixed_check(a, end, thresh, c->s));
                 c->launches += 1;
             }
             processed = end;

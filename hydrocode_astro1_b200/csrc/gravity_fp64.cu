@@ -560,13 +560,7 @@ cudaError_t grav_sor_pass64(const GravArgs &a, const double *in, double *out, in
     static std::atomic<unsigned long long> attr_set{0};
     cudaError_t e = set_smem_once(attr_set, (const void *)kern, (int)sm);
     if (e != cudaSuccess) return e;
-    SorCoef<double> cf;
-    cf.ix2 = 1.0 / (a.g.dx * a.g.dx);
-    cf.iy2 = 1.0 / (a.g.dy * a.g.dy);
-    cf.iz2 = 1.0 / (a.g.dz * a.g.dz);
-    cf.fpg = 4.0 * M_PI * a.G;
-    cf.fac = 2.0 * (cf.ix2 + cf.iy2 + cf.iz2);
-    cf.om = a.omega;
+    const SorCoef<double> cf = sor_coef64(a.g.dx, a.g.dy, a.g.dz, a.G, a.omega);
     const int tj = (a.g.ny + WF64_TJ - 1) / WF64_TJ, tk = (a.g.nz + WF64_TK - 1) / WF64_TK;
     const int nint = a.g.nx - 2;
     // about 3 waves of 4 CTAs per SM; at least 16 planes per chunk
@@ -597,6 +591,7 @@ cudaError_t grav_sor_pass64(const GravArgs &a, const double *in, double *out, in
 // ---------------------------------------------------------------------------
 // Colour-split SOR (the default FP64 solve for nz >= 3)
 // ---------------------------------------------------------------------------
+#include "sor_resident.cuh"
 #include "sor_split.cuh"
 
 namespace hc {
@@ -632,16 +627,30 @@ cudaError_t grav_unsplit(const GravArgs &a, const double *phs, cudaStream_t s)
     return cudaGetLastError();
 }
 
+static SorCoef<double> sor_coef64(const GravArgs &a) { return sor_coef64(a.g.dx, a.g.dy, a.g.dz, a.G, a.omega); }
+
 cudaError_t grav_sor_split(const GravArgs &a, double *phs, const double *rhs, int colour, int iter, cudaStream_t s)
 {
-    SorCoef<double> cf;
-    cf.ix2 = 1.0 / (a.g.dx * a.g.dx);
-    cf.iy2 = 1.0 / (a.g.dy * a.g.dy);
-    cf.iz2 = 1.0 / (a.g.dz * a.g.dz);
-    cf.fpg = 4.0 * M_PI * a.G;
-    cf.fac = 2.0 * (cf.ix2 + cf.iy2 + cf.iz2);
-    cf.om = a.omega;
-    return launch_sor_split<double, double>(phs, rhs, make_split(a.g), cf, colour, a.res, iter, a.tol, a.sc, s);
+    return launch_sor_split<double, double>(phs, rhs, make_split(a.g), sor_coef64(a), colour, a.res, iter, a.tol, a.sc,
+                                            s);
+}
+
+bool grav_resident_plan(const Geom &g, size_t elem, ResPlan *out)
+{
+    int dev = 0, sms = 0, optin = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess)
+        return false;
+    return coop && optin > RS_STATIC && res_plan(g, elem, sms, (size_t)(optin - RS_STATIC), out);
+}
+
+cudaError_t grav_sor_resident(const GravArgs &a, double *phs, const double *rhs, const ResPlan &p, void *exch,
+                              unsigned epoch, int it0, int n, cudaStream_t s)
+{
+    return run_resident<double>(p, phs, rhs, make_split(a.g), sor_coef64(a), exch, epoch, a.res, it0, n, a.tol, a.sc,
+                                s);
 }
 
 }  // namespace hc

@@ -15,6 +15,7 @@
 
 #include "hc_internal.cuh"
 #include "hc_math.cuh"
+#include "sor_resident.cuh"
 #include "sor_split.cuh"
 #include "sor_split_tma.cuh"
 #include "sor_wave_split.cuh"
@@ -784,8 +785,7 @@ static cudaError_t sweep_tma(float *base, const float *src, const Split &sp, con
                            tl, cf, colour, res, iter, thresh, sc);
 }
 
-cudaError_t mixed_sor32_split(const GravArgs &a, float *e32, const float *r32, int colour, int iter,
-                              double thresh, cudaStream_t s)
+static SorCoef<float> sor_coef32(const GravArgs &a)
 {
     const MixConst mc = mix_const(a);
     SorCoef<float> cf;
@@ -793,6 +793,20 @@ cudaError_t mixed_sor32_split(const GravArgs &a, float *e32, const float *r32, i
     cf.cy = mc.cy;
     cf.cz = mc.cz;
     cf.om = mc.om;
+    return cf;
+}
+
+cudaError_t mixed_sor32_resident(const GravArgs &a, float *e32, const float *r32, const ResPlan &p, void *exch,
+                                 unsigned epoch, int it0, int n, double thresh, cudaStream_t s)
+{
+    return run_resident<float>(p, e32, r32, make_split(a.g), sor_coef32(a), exch, epoch, a.res, it0, n, thresh, a.sc,
+                               s);
+}
+
+cudaError_t mixed_sor32_split(const GravArgs &a, float *e32, const float *r32, int colour, int iter,
+                              double thresh, cudaStream_t s)
+{
+    const SorCoef<float> cf = sor_coef32(a);
     const Split sp = make_split(a.g);
     if (a.sweep_kind == 1 && sp.H % 4 == 0 && sp.H <= stma::HMAX && sp.nx >= 3 && sp.ny >= 3 &&
         ((uintptr_t)e32 | (uintptr_t)r32) % 16 == 0 && sp.cs % 4 == 0) {

@@ -247,6 +247,20 @@ cudaError_t grav_split_fields(const GravArgs &a, double *phs, double *rhs, cudaS
 cudaError_t grav_split_boundary(const GravArgs &a, double *phs, cudaStream_t s);
 cudaError_t grav_unsplit(const GravArgs &a, const double *phs, cudaStream_t s);
 cudaError_t grav_sor_split(const GravArgs &a, double *phs, const double *rhs, int colour, int iter, cudaStream_t s);
+// many iterations per launch on grids that fit the SMs' shared memory
+// (sor_resident.cuh): the blocks of a grid for words of `elem` bytes (false:
+// it does not fit), and iterations it0 .. it0 + n - 1 until the stop test
+// (the launch sets done / last_iter).  exch: plan.exch_bytes of device memory,
+// zeroed once and kept; epoch: a number that advances by 4 n + 16 per launch
+struct ResPlan {
+    int gi = 0, gj = 0, BI = 0, BJ = 0, Hp = 0;
+    size_t smem = 0, exch_bytes = 0;
+};
+bool grav_resident_plan(const Geom &g, size_t elem, ResPlan *out);
+cudaError_t grav_sor_resident(const GravArgs &a, double *phs, const double *rhs, const ResPlan &p, void *exch,
+                              unsigned epoch, int it0, int n, cudaStream_t s);
+cudaError_t mixed_sor32_resident(const GravArgs &a, float *e32, const float *r32, const ResPlan &p, void *exch,
+                                 unsigned epoch, int it0, int n, double thresh, cudaStream_t s);
 cudaError_t mixed_sor32_pass(const GravArgs &a, const float *in, float *out, const float *r32, int iter0,
                              int depth, double thresh, cudaStream_t s);
 }  // namespace hc

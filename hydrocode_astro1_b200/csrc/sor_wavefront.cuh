@@ -21,24 +21,71 @@
 // max and one atomic per CTA into that iteration's slot.  A pass starts only
 // if the previous iteration's slot is not below the stop threshold.
 #pragma once
+#include <cmath>
+
 #include "hc_internal.cuh"
 #include "hc_math.cuh"
 
 namespace hc {
 
 template <typename T> struct SorCoef;
+// x / y, kept out of line: only operands outside quotient()'s range need it
+static __device__ __noinline__ double sor_divide(double x, double y) { return x / y; }
+
 template <> struct SorCoef<double> {
     double ix2, iy2, iz2, fpg, fac, om;
+    double rh, rl;     // 1 / fac as RN(1 / fac) + remainder
+    unsigned span;     // exponents for which quotient() multiplies (0: always divides)
+
+    // RN(x / fac) with the divisor known in advance: q = RN(x rh + RN(x rl)) is
+    // within one ulp of x / fac, the remainder x - q fac is exact, and one
+    // correction with RN(1 / fac) rounds correctly (P. Markstein, "Computation of
+    // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+    // Dev. 34, 1990; N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
+    // correctly rounded floating-point division when the divisor is known in
+    // advance", IEEE Trans. Comput. 53, 2004).  |x| in [2^-900, 2^900) keeps every
+    // term normal; other x (zero, tiny, huge, not finite) divide.  The quotient
+    // costs 4 FP64 operations; the division was over a third of an update's.
+    __device__ __forceinline__ bool out_of_range(double x) const
+    {
+        return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 900u) << 20) >= span;
+    }
+    __device__ __forceinline__ double quotient_in_range(double x) const
+    {
+        const double q = __fma_rn(x, rh, __dmul_rn(x, rl));
+        return __fma_rn(__fma_rn(-q, fac, x), rh, q);
+    }
+    __device__ __forceinline__ double quotient(double x) const
+    {
+        return out_of_range(x) ? sor_divide(x, fac) : quotient_in_range(x);
+    }
     __device__ __forceinline__ double update(double old, double xm, double xp, double ym, double yp,
                                              double zm, double zp, double src, double &r) const
     {
         // gravity_solver_3d.c:654-671, operand order kept
         double lap = (xm + xp) * ix2 + (ym + yp) * iy2 + (zm + zp) * iz2;
-        double nw = (lap - fpg * src) / fac;
+        double nw = quotient(lap - fpg * src);
         r = fabs(nw - old);
         return old + om * (nw - old);
     }
 };
+
+inline SorCoef<double> sor_coef64(double dx, double dy, double dz, double G, double omega)
+{
+    SorCoef<double> c;
+    c.ix2 = 1.0 / (dx * dx);
+    c.iy2 = 1.0 / (dy * dy);
+    c.iz2 = 1.0 / (dz * dz);
+    c.fpg = 4.0 * M_PI * G;
+    c.fac = 2.0 * (c.ix2 + c.iy2 + c.iz2);
+    c.om = omega;
+    c.rh = 1.0 / c.fac;
+    c.rl = std::fma(-c.rh, c.fac, 1.0) / c.fac;
+    int ex = 0;
+    const double m = std::frexp(c.fac, &ex);   // fac = m 2^ex; an all-ones m has no correctly rounded 1 / fac to use
+    c.span = std::isfinite(c.fac) && ex > -100 && ex < 100 && m != 1.0 - 0x1p-53 ? 1800u << 20 : 0u;
+    return c;
+}
 // FP32 correction sweep: e_GS = cx (e_x- + e_x+) + cy (..) + cz (..) + delta.
 // The multiply-adds are written out (fmaf), so every FP32 sweep kernel --
 // scalar, vector, streaming and the two-iteration pass -- rounds each update
