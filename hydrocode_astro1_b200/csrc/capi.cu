@@ -100,6 +100,8 @@ struct hc_ctx {
     double *scratch;
     long long scratch_len;
     double *mom;
+    void *seq;                   // work of the sequential moments
+    int seq_tried;
     // scalars
     DevScalars *sc;
     DevScalars *hsc;             // pinned mirror
@@ -233,7 +235,7 @@ static void free_ctx(hc_ctx *c)
     cudaFree(c->phs); cudaFree(c->rhs); cudaFree(c->plm); cudaFree(c->slab_buf);
     cudaFree(c->e32); cudaFree(c->r32); cudaFree(c->e32b); cudaFree(c->exch);
     cudaFree(c->gx); cudaFree(c->gy); cudaFree(c->gz);
-    cudaFree(c->res); cudaFree(c->scratch); cudaFree(c->mom); cudaFree(c->cons_part);
+    cudaFree(c->res); cudaFree(c->seq); cudaFree(c->scratch); cudaFree(c->mom); cudaFree(c->cons_part);
     cudaFree(c->sc); cudaFree(c->stage);
     if (c->hsc) cudaFreeHost(c->hsc);
     if (c->hdt) cudaFreeHost(c->hdt);
@@ -499,6 +501,20 @@ extern "C" int hc_get_state_soa(hc_ctx *c, double *q)
 }
 
 // ---------------------------------------------------------------- gravity
+// Work of the sequential moments, once per context; without room for it they
+// are added cell by cell.
+static void *ensure_seq(hc_ctx *c)
+{
+    if (!c->seq && !c->seq_tried) {
+        c->seq_tried = 1;
+        if (cudaMalloc(&c->seq, grav_seq_bytes(c->g)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            c->seq = nullptr;
+        }
+    }
+    return c->seq;
+}
+
 static GravArgs grav_args(hc_ctx *c, const double *rho, const float *rho32)
 {
     GravArgs a;
@@ -544,14 +560,16 @@ static int grav_boundary_values(hc_ctx *c, const GravArgs &a)
     return HC_OK;
 }
 
-static int grav_moments(hc_ctx *c, const GravArgs &a)
+static int grav_moments(hc_ctx *c, const GravArgs &a0)
 {
+    GravArgs a = a0;
     if (a.grav_bc != 1) return HC_OK;
+    if (a.lmax == 0 && a.moment_order == HC_MOMENTS_SEQUENTIAL && a.rho) a.seq = ensure_seq(c);
     FamTimer t(c, FAM_MOM);
     if (a.lmax == 0) {
         if (a.moment_order == HC_MOMENTS_SEQUENTIAL && a.rho) {
             CK(grav_moments_sequential(a, c->s));
-            c->launches += 1;
+            c->launches += a.seq ? 16 : 4;
         } else {
             CK(grav_moments_tree(a, c->s));
             c->launches += 4;
@@ -1591,6 +1609,7 @@ extern "C" int hc_slab_moments(hc_ctx *c, int pass, double *buf)
         FamTimer t(c, FAM_MOM);
         if (slab_sequential(c)) {
             CK(cudaMemcpyAsync(c->slab_buf, buf, count * sizeof(double), cudaMemcpyHostToDevice, c->s));
+            a.seq = ensure_seq(c);
             CK(grav_moments_seq_slab(a, pass, c->slab_buf, c->s));
         } else if (c->cfg.lmax == 0) {
             CK(grav_moments_tree_parts(a, pass, c->slab_buf, c->s));

@@ -4,7 +4,7 @@
 //
 //   moments      M, centre of mass and the Cartesian quadrupole Q_ij over
 //                cells with rho > 0 (:164-262).  HC_MOMENTS_SEQUENTIAL sums in
-//                the reference's (i,j,k) order on one CTA -- bit-exact;
+//                the reference's (i,j,k) order -- bit-exact (seq_* below);
 //                HC_MOMENTS_TREE is a fixed-shape (deterministic) tree.
 //   boundary     monopole + quadrupole potential on the six faces (:302-498),
 //                each face cell given the value of the face loop that writes
@@ -46,21 +46,13 @@ __device__ __forceinline__ double block_max_d(double v)
 }
 
 // ---------------------------------------------------------------- moments
-constexpr int SEQ_CH = 1024;
-constexpr int SEQ_NT = 256;
-
-// Bit-exact moments: terms per cell are formed in parallel into shared
-// memory, then one thread per accumulator adds them in cell order.
-
-// The terms of cell c: pass 0 (dm, dm x, dm y, dm z), pass 1 the quadrupole
-// terms about com (gravity_solver_3d.c:181-190, :236-255); zero where rho <= 0.
-__device__ __forceinline__ void seq_terms(const GravArgs &a, int pass, long long c, const double *com, double *t)
+// The terms of a cell of density r: pass 0 (dm, dm x, dm y, dm z), pass 1 the
+// quadrupole terms about com (gravity_solver_3d.c:181-190, :236-255); zero
+// where r <= 0.
+__device__ __forceinline__ void seq_terms(const Geom &g, int pass, double r, int i, int j, int k, const double *com,
+                                          double *t)
 {
-    const Geom &g = a.g;
-    const double r = a.rho ? a.rho[c] : (double)a.rho32[c];
     if (!(r > 0.0)) return;
-    const long long snz = g.nz, sjk = (long long)g.ny * g.nz;
-    const int i = (int)(c / sjk), j = (int)((c / snz) % g.ny), k = (int)(c % snz);
     const double dm = r * (g.dx * g.dy * g.dz);
     if (pass == 0) {
         double x = g.xmin + (i + g.ioff + 0.5) * g.dx;
@@ -84,29 +76,9 @@ __device__ __forceinline__ void seq_terms(const GravArgs &a, int pass, long long
     }
 }
 
-// One pass over the cells [c0, c1) in order: thread q < nv returns acc plus
-// term q of every cell, added one by one.
-__device__ double seq_pass(const GravArgs &a, int pass, long long c0, long long c1, const double *com,
-                           double *term, double acc)
+__device__ __forceinline__ double seq_density(const GravArgs &a, long long c)
 {
-    const int tid = threadIdx.x;
-    const int nv = pass == 0 ? 4 : 9;
-    for (long long base = c0; base < c1; base += SEQ_CH) {
-        for (int e = tid; e < SEQ_CH; e += SEQ_NT) {
-            const long long c = base + e;
-            double t[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-            if (c < c1) seq_terms(a, pass, c, com, t);
-            for (int q = 0; q < nv; q++) term[q * SEQ_CH + e] = t[q];
-        }
-        __syncthreads();
-        if (tid < nv) {
-            const double *tt = term + tid * SEQ_CH;
-            const int m = (int)min((long long)SEQ_CH, c1 - base);
-            for (int e = 0; e < m; e++) acc += tt[e];
-        }
-        __syncthreads();
-    }
-    return acc;
+    return a.rho ? a.rho[c] : (double)a.rho32[c];
 }
 
 __device__ __forceinline__ void centre_of_mass(const Geom &g, const double *acc, double *out)
@@ -122,33 +94,361 @@ __device__ __forceinline__ void centre_of_mass(const Geom &g, const double *acc,
     }
 }
 
-__global__ void __launch_bounds__(SEQ_NT) moments_seq_kernel(GravArgs a)
+// The sums in the reference's cell order, bit for bit, in parallel.
+//
+// Let r_i = RN(r_(i-1) + t_i) be the partial sums of a run of cells from a
+// start g, u_i the unit in the last place of r_i and U the largest of them.
+// From g + d, d a multiple of 2 U, every partial sum is r_i + d, as long as
+// r_i and r_i + d lie in the same binade throughout: d is a multiple of every
+// u_i, an even one, so it passes through each rounding, halves included.  So
+// a run that was added up from a guess gives the result for any start that
+// differs from it by such a d, smaller than the least distance of an r_i to
+// the ends of its binade (the margin).
+//   seq_totals   plain sums of the runs (32 .. 256 cells), added up by
+//                seq_prefix to estimates of the sum at each run's start
+//   seq_first    every run added up from its estimate
+//   seq_second   again from g = (the result of the run before) + the multiple
+//                of U nearest to the estimate, and from g + U: a run forgets
+//                its start's bits below its own U, so the result before has
+//                the right low bits although its high ones are a guess
+//   seq_groups   the same twice for groups of 32 runs (first, then second), a
+//                run taken by its record where that holds, else cell by cell
+//   seq_walk     from the true sum over the groups; a group whose record does
+//                not hold is taken run by run, a run cell by cell
+// A guess only decides whether a record can be used; what is used is checked
+// against the sum itself.  The records hold for sums that keep their sign as
+// for those that return to zero in every row (z and the mixed moments of a
+// centred box), where the binade changes every few cells.
+// Bound: a chain of dependent FP64 additions.  One CTA adding cell by cell (17
+// cycles a cell) took 4.65 ms at 64^3, 35.8 ms at 128^3 and 317 ms at 256^3 for both
+// passes; this takes 0.45-0.54, 1.3-1.8 and 7-17 ms, the last walk and, at
+// 256^3, the terms' arithmetic being the most of it.
+constexpr int SEQ_GRP = 32;        // runs of a group
+constexpr int SEQ_DIRECT = 14000;  // cells below which the sums are added cell by cell: 24^3 takes 230 us,
+                                   // the records' sixteen launches 225-265 us at 26^3
+constexpr double SEQ_ALL = 1e300;  // the margin before the first term
+
+struct SeqRecs {
+    double *g, *out, *margin;   // [variant][sum][record]
+    int *ue;                    // exponent of U
+    long long n;                // records per sum
+};
+struct SeqWork {
+    double *pre;                // per run: plain total, then the estimate at its start
+    double *out1[2];            // first results of runs / groups
+    int *ue1[2];
+    SeqRecs lev[2];             // runs, groups
+    int G;                      // cells of a run
+};
+
+// Partial sums: the sum, the largest unit and the least distance to a binade's end.
+struct SeqSum {
+    double acc, margin;
+    int ue;                     // biased exponent of the largest partial sum
+    __device__ __forceinline__ void add(double t)
+    {
+        if (t == 0.0) return;   // acc + 0 is acc
+        acc += t;
+        const int hi = __double2hiint(acc) & 0x7fffffff, e = hi >> 20;
+        const double m = fabs(acc), bin = __hiloint2double(e << 20, 0);
+        margin = fmin(margin, e > 60 && e < 2000 ? fmin(m - bin, 2.0 * bin - m) : 0.0);
+        ue = max(ue, e);
+    }
+};
+__device__ __forceinline__ double seq_unit(int ue) { return __hiloint2double((ue - 52) << 20, 0); }
+
+// The sum after a record, from s: exactly the start, or 2 U-multiples away
+// from it within the margin.
+__device__ __forceinline__ bool seq_use(SeqSum &s, double g, double out, double margin, int ue)
 {
-    extern __shared__ double term[];   // 9 x SEQ_CH
-    __shared__ double accs[9];
-    __shared__ double mc[4];
-    const int tid = threadIdx.x;
-    const long long n = a.g.n;
-    double acc = seq_pass(a, 0, 0, n, nullptr, term, 0.0);
-    if (tid < 4) accs[tid] = acc;
-    __syncthreads();
-    if (tid == 0) centre_of_mass(a.g, accs, mc);
-    __syncthreads();
-    acc = seq_pass(a, 1, 0, n, mc + 1, term, 0.0);
-    if (tid < 4) a.sc->moments[tid] = mc[tid];
-    if (tid < 9) a.sc->moments[4 + tid] = acc;
+    if (margin >= SEQ_ALL) return true;   // no term but zeros
+    const double d = s.acc - g;
+    if (d != 0.0) {
+        if (!(fabs(d) < margin)) return false;
+        // d exact (two-sum), and a multiple of 2 U
+        const double bb = s.acc - d;
+        if (((s.acc - (d + bb)) + (bb - g)) != 0.0) return false;
+        const double q = d * __hiloint2double((2097 - ue) << 20, 0);   // d / (2 U), 2 U = 2^(ue - 1074)
+        if (!(fabs(q) < 0x1p50) || q != rint(q)) return false;
+    }
+    s.acc = out + d;
+    s.margin = fmin(s.margin, margin - fabs(d));
+    s.ue = max(s.ue, ue);
+    return true;
 }
 
-// A slab's share of the sequential sums: the own planes, continuing acc.
-__global__ void __launch_bounds__(SEQ_NT) moments_seq_slab_kernel(GravArgs a, int pass, double *acc)
+// term q of pass PASS of cell c
+template <int PASS>
+__device__ __forceinline__ double seq_term(const GravArgs &a, int q, double r, int i, int j, int k, const double *com)
 {
-    extern __shared__ double term[];
-    const int tid = threadIdx.x;
-    const int nv = pass == 0 ? 4 : 9;
-    const long long sjk = (long long)a.g.ny * a.g.nz;
-    double v = tid < nv ? acc[tid] : 0.0;
-    v = seq_pass(a, pass, a.g.olo * sjk, a.g.ohi * sjk, a.sc->moments + 1, term, v);
-    if (tid < nv) acc[tid] = v;
+    constexpr int NV = PASS ? 9 : 4;
+    double t[9] = {};
+    seq_terms(a.g, PASS, r, i, j, k, com, t);
+    double v = t[0];
+#pragma unroll
+    for (int x = 1; x < NV; x++) v = q == x ? t[x] : v;
+    return v;
+}
+
+// f(term q) for the cells [c, c + n) below c1, in order
+template <int PASS, typename F>
+__device__ __forceinline__ void seq_cells(const GravArgs &a, int q, long long c, int n, long long c1,
+                                          const double *com, F f)
+{
+    const Geom &g = a.g;
+    const int sjk = g.ny * g.nz;
+    int i = (int)(c / sjk), rest = (int)(c % sjk), j = rest / g.nz, k = rest % g.nz;
+    n = (int)min((long long)n, c1 - c);
+#pragma unroll 4
+    for (int x = 0; x < n; x++) {
+        f(seq_term<PASS>(a, q, seq_density(a, c + x), i, j, k, com));
+        if (++k == g.nz) {
+            k = 0;
+            if (++j == g.ny) {
+                j = 0;
+                i++;
+            }
+        }
+    }
+}
+
+// the plain total of every run (blockIdx.y: the sum)
+template <int PASS>
+__global__ void __launch_bounds__(128) seq_totals_kernel(GravArgs a, long long c0, long long c1, SeqWork w)
+{
+    const int q = blockIdx.y;
+    const long long r = blockIdx.x * 128LL + threadIdx.x, n = w.lev[0].n;
+    if (r >= n) return;
+    const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
+    double s = 0.0;
+    seq_cells<PASS>(a, q, c0 + r * w.G, w.G, c1, com, [&](double t) { s += t; });
+    w.pre[q * n + r] = s;
+}
+
+// totals -> estimates of the sum at each run's start (CTA per sum, a stretch
+// of the runs per thread)
+__global__ void __launch_bounds__(1024) seq_prefix_kernel(SeqWork w, const double *acc)
+{
+    const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const long long n = w.lev[0].n, per = (n + 1023) / 1024, i0 = tid * per, i1 = min(n, i0 + per);
+    double *p = w.pre + q * n;
+    double s = 0.0;
+    for (long long i = i0; i < i1; i++) s += p[i];
+    __shared__ double ws[32];
+    double x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[tid >> 5] = x;
+    __syncthreads();
+    double base = acc[q] + (x - s);
+    for (int v = 0; v < tid >> 5; v++) base += ws[v];
+    for (long long i = i0; i < i1; i++) {
+        const double v = p[i];
+        p[i] = base;
+        base += v;
+    }
+}
+
+// runs from their estimates
+template <int PASS>
+__global__ void __launch_bounds__(128) seq_first_kernel(GravArgs a, long long c0, long long c1, SeqWork w)
+{
+    const int q = blockIdx.y;
+    const long long r = blockIdx.x * 128LL + threadIdx.x, n = w.lev[0].n;
+    if (r >= n) return;
+    const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
+    SeqSum s = { w.pre[q * n + r], SEQ_ALL, 0 };
+    seq_cells<PASS>(a, q, c0 + r * w.G, w.G, c1, com, [&](double t) { s.add(t); });
+    w.out1[0][q * n + r] = s.acc;
+    w.ue1[0][q * n + r] = s.ue;
+}
+
+// the guess for record r of a level: the low bits of the result before it,
+// the high bits of the estimate; variant 1 one U further
+__device__ __forceinline__ double seq_guess(const double *out1, int ue, long long at, long long r, double est,
+                                            double first, int variant)
+{
+    const double U = ue > 60 ? seq_unit(ue) : 0.0;
+    double g = first;
+    if (r > 0) {
+        const double p = out1[at - 1];
+        g = U > 0.0 ? p + rint((est - p) / U) * U : p;
+    }
+    return variant ? g + U : g;
+}
+
+// runs from their guesses (blockIdx.z: the variant)
+template <int PASS>
+__global__ void __launch_bounds__(128) seq_second_kernel(GravArgs a, long long c0, long long c1, SeqWork w,
+                                                         const double *acc)
+{
+    const int q = blockIdx.y, v = blockIdx.z;
+    const long long r = blockIdx.x * 128LL + threadIdx.x, n = w.lev[0].n;
+    if (r >= n) return;
+    const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
+    const long long at = q * n + r;
+    const double g = seq_guess(w.out1[0], w.ue1[0][at], at, r, w.pre[at], acc[q], v);
+    SeqSum s = { g, SEQ_ALL, 0 };
+    seq_cells<PASS>(a, q, c0 + r * w.G, w.G, c1, com, [&](double t) { s.add(t); });
+    const SeqRecs &o = w.lev[0];
+    const long long x = (long long)v * (PASS ? 9 : 4) * n + at;
+    o.g[x] = g;
+    o.out[x] = s.acc;
+    o.margin[x] = s.margin;
+    o.ue[x] = s.ue;
+}
+
+// 32 records of one sum, both variants, one per lane
+struct SeqBatch {
+    double g[2], out[2], margin[2];
+    int ue[2];
+    __device__ __forceinline__ void fetch(const SeqRecs &r, int nv, int q, long long at)
+    {
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+            const long long x = ((long long)v * nv + q) * r.n + min(at, r.n - 1);
+            g[v] = r.g[x];
+            out[v] = r.out[x];
+            margin[v] = r.margin[x];
+            ue[v] = r.ue[x];
+        }
+    }
+    // s after lane j's record (the same in every lane)
+    __device__ __forceinline__ bool use(int j, SeqSum &s) const
+    {
+#pragma unroll
+        for (int v = 0; v < 2; v++)
+            if (seq_use(s, __shfl_sync(0xffffffffu, g[v], j), __shfl_sync(0xffffffffu, out[v], j),
+                        __shfl_sync(0xffffffffu, margin[v], j), __shfl_sync(0xffffffffu, ue[v], j)))
+                return true;
+        return false;
+    }
+};
+
+// A warp takes sum q over the runs [r0, r1), at most SEQ_GRP of them
+template <int PASS>
+__device__ __forceinline__ void seq_runs(const GravArgs &a, long long c0, long long c1, const SeqWork &w, int q,
+                                         long long r0, long long r1, const double *com, SeqSum &s)
+{
+    const int lane = threadIdx.x & 31;
+    SeqBatch b;
+    b.fetch(w.lev[0], PASS ? 9 : 4, q, r0 + lane);
+    for (int j = 0; j < (int)(r1 - r0); j++) {
+        if (b.use(j, s)) continue;
+        const long long c = c0 + (r0 + j) * w.G;
+        for (int x = 0; x < w.G; x += 32) {   // 32 terms at a time, then their chain
+            double t = 0.0;
+            seq_cells<PASS>(a, q, c + x + lane, 1, c1, com, [&](double v) { t = v; });
+#pragma unroll
+            for (int k = 0; k < 32; k++) s.add(__shfl_sync(0xffffffffu, t, k));
+        }
+    }
+}
+
+// groups (warp per group, sum blockIdx.y): first from the first run's guess,
+// then (second) from the guesses made of the first results, as for the runs
+template <int PASS>
+__global__ void __launch_bounds__(32) seq_groups_kernel(GravArgs a, long long c0, long long c1, SeqWork w,
+                                                        const double *acc, int second)
+{
+    const int q = blockIdx.y, v = blockIdx.z;
+    const long long h = blockIdx.x, n0 = w.lev[0].n, n = w.lev[1].n, r0 = h * SEQ_GRP;
+    const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
+    const long long at = q * n + h;
+    const double est = w.lev[0].g[q * n0 + r0];
+    const double g = second ? seq_guess(w.out1[1], w.ue1[1][at], at, h, est, acc[q], v) : est;
+    SeqSum s = { g, SEQ_ALL, 0 };
+    seq_runs<PASS>(a, c0, c1, w, q, r0, min(n0, r0 + SEQ_GRP), com, s);
+    if (threadIdx.x != 0) return;
+    if (!second) {
+        w.out1[1][at] = s.acc;
+        w.ue1[1][at] = s.ue;
+        return;
+    }
+    const SeqRecs &o = w.lev[1];
+    const long long x = (long long)v * (PASS ? 9 : 4) * n + at;
+    o.g[x] = g;
+    o.out[x] = s.acc;
+    o.margin[x] = s.margin;
+    o.ue[x] = s.ue;
+}
+
+// The cells [c0, c1) one by one, by the whole CTA: the terms of a stretch of
+// cells in parallel into shared memory, then thread q < NV adds term q of each
+// to acc, in order.
+constexpr int SEQ_CH = 448, SEQ_ST = SEQ_CH + 1;   // an odd stride: the sums' terms lie in different banks
+template <int PASS>
+__device__ double seq_chain(const GravArgs &a, long long c0, long long c1, const double *com, double *term, double acc)
+{
+    constexpr int NV = PASS ? 9 : 4;
+    const Geom &g = a.g;
+    const int tid = threadIdx.x, sjk = g.ny * g.nz;
+    for (long long b = c0; b < c1; b += SEQ_CH) {
+        const int m = (int)min((long long)SEQ_CH, c1 - b);
+        for (int e = tid; e < m; e += blockDim.x) {
+            const long long c = b + e;
+            const int i = (int)(c / sjk), rest = (int)(c % sjk);
+            double t[9] = {};
+            seq_terms(g, PASS, seq_density(a, c), i, rest / g.nz, rest % g.nz, com, t);
+#pragma unroll
+            for (int q = 0; q < NV; q++) term[q * SEQ_ST + e] = t[q];
+        }
+        __syncthreads();
+        if (tid < NV) {
+            const double *tt = term + tid * SEQ_ST;
+#pragma unroll 16
+            for (int e = 0; e < m; e++) acc += tt[e];
+        }
+        __syncthreads();
+    }
+    return acc;
+}
+
+// Both passes in one launch, cell by cell: below SEQ_DIRECT cells the chain
+// is shorter than the launches of the records.
+__global__ void __launch_bounds__(288) seq_direct_kernel(GravArgs a)
+{
+    __shared__ double term[9 * SEQ_ST], acc[9], mc[4];
+    const int q = threadIdx.x;
+    double v = seq_chain<0>(a, 0, a.g.n, nullptr, term, 0.0);
+    if (q < 4) acc[q] = v;
+    __syncthreads();
+    if (q == 0) centre_of_mass(a.g, acc, mc);
+    __syncthreads();
+    v = seq_chain<1>(a, 0, a.g.n, mc + 1, term, 0.0);
+    if (q < 9) a.sc->moments[4 + q] = v;
+    if (q < 4) a.sc->moments[q] = mc[q];
+}
+
+// Warp q takes sum q over the cells [c0, c1), from acc[q] to acc[q].  Without
+// work memory (w.G == 0) cell by cell.
+template <int PASS>
+__global__ void __launch_bounds__(PASS ? 288 : 128) seq_walk_kernel(GravArgs a, long long c0, long long c1,
+                                                                    SeqWork w, double *acc)
+{
+    __shared__ double term[(PASS ? 9 : 4) * SEQ_ST];
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
+    if (!w.G) {
+        const int t = threadIdx.x;
+        const double v = seq_chain<PASS>(a, c0, c1, com, term, t < (PASS ? 9 : 4) ? acc[t] : 0.0);
+        if (t < (PASS ? 9 : 4)) acc[t] = v;
+        return;
+    }
+    SeqSum s = { acc[q], SEQ_ALL, 0 };   // the same in every lane
+    {
+        SeqBatch b;
+        for (long long h = 0; h < w.lev[1].n; h++) {
+            const int j = (int)(h % 32);
+            if (j == 0) b.fetch(w.lev[1], PASS ? 9 : 4, q, h + lane);
+            if (!b.use(j, s))
+                seq_runs<PASS>(a, c0, c1, w, q, h * SEQ_GRP, min(w.lev[0].n, (h + 1) * SEQ_GRP), com, s);
+        }
+    }
+    if (lane == 0) acc[q] = s.acc;
 }
 
 __global__ void moments_seq_set_kernel(GravArgs a, int pass, const double *acc)
@@ -174,7 +474,8 @@ __global__ void __launch_bounds__(TREE_NT) moments_tree_partial(GravArgs a, int 
     double acc[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
     for (long long c = c0 + threadIdx.x; c < c0 + sjk; c += TREE_NT) {
         double t[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-        seq_terms(a, pass, c, com, t);
+        const int r = (int)(c - c0);
+        seq_terms(g, pass, seq_density(a, c), g.olo + blockIdx.x, r / g.nz, r % g.nz, com, t);
         for (int q = 0; q < nv; q++) acc[q] += t[q];
     }
     __shared__ double red[TREE_NT / 32][9];
@@ -421,24 +722,93 @@ inline int grid_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 
 }  // namespace
 
-cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s)
+// Where the records of a pass over n cells lie in the work buffer.  Runs of
+// 32 cells for small grids (a chain is short), up to 256 for large ones (the
+// last walk is over n / (32 G) groups).
+static SeqWork seq_layout(long long n0, void *buf, size_t *bytes)
 {
-    const size_t sm = 9 * SEQ_CH * sizeof(double);
-    static std::atomic<unsigned long long> attr_set{0};
-    cudaError_t e = set_smem_once(attr_set, (const void *)moments_seq_kernel, (int)sm);
-    if (e != cudaSuccess) return e;
-    moments_seq_kernel<<<1, SEQ_NT, sm, s>>>(a);
+    SeqWork w;
+    w.G = 0;
+    char *p = static_cast<char *>(buf);
+    auto take = [&](long long items, size_t each) {
+        char *r = p;
+        p += (items * each + 255) / 256 * 256;
+        return r;
+    };
+    w.pre = reinterpret_cast<double *>(take(9 * n0, 8));
+    for (int l = 0; l < 2; l++) {
+        const long long k = l ? (n0 + SEQ_GRP - 1) / SEQ_GRP : n0;
+        w.out1[l] = reinterpret_cast<double *>(take(9 * k, 8));
+        w.ue1[l] = reinterpret_cast<int *>(take(9 * k, 4));
+        w.lev[l].g = reinterpret_cast<double *>(take(18 * k, 8));
+        w.lev[l].out = reinterpret_cast<double *>(take(18 * k, 8));
+        w.lev[l].margin = reinterpret_cast<double *>(take(18 * k, 8));
+        w.lev[l].ue = reinterpret_cast<int *>(take(18 * k, 4));
+        w.lev[l].n = k;
+    }
+    if (bytes) *bytes = (size_t)(p - static_cast<char *>(buf));
+    return w;
+}
+
+static SeqWork seq_work(long long n, void *buf)
+{
+    int G = 32;
+    while (G < 256 && n / G > 4096) G *= 2;
+    SeqWork w = seq_layout((n + G - 1) / G, buf, nullptr);
+    w.G = G;
+    return w;
+}
+
+size_t grav_seq_bytes(const Geom &g)
+{
+    // the most runs of any range of the grid: 4097 of fewer than 256 cells, or n / 256
+    size_t b = 0;
+    seq_layout(std::max<long long>(g.n / 256 + 1, std::min<long long>(g.n / 32 + 1, 4097)), nullptr, &b);
+    return b;
+}
+
+template <int PASS>
+static cudaError_t seq_run(const GravArgs &a, long long c0, long long c1, double *acc, cudaStream_t s)
+{
+    constexpr int NV = PASS ? 9 : 4;
+    SeqWork w = {};
+    if (a.seq && c1 - c0 >= SEQ_DIRECT) {
+        w = seq_work(c1 - c0, a.seq);
+        const unsigned nb = (unsigned)((w.lev[0].n + 127) / 128), ng = (unsigned)w.lev[1].n;
+        seq_totals_kernel<PASS><<<dim3(nb, NV), 128, 0, s>>>(a, c0, c1, w);
+        seq_prefix_kernel<<<NV, 1024, 0, s>>>(w, acc);
+        seq_first_kernel<PASS><<<dim3(nb, NV), 128, 0, s>>>(a, c0, c1, w);
+        seq_second_kernel<PASS><<<dim3(nb, NV, 2), 128, 0, s>>>(a, c0, c1, w, acc);
+        seq_groups_kernel<PASS><<<dim3(ng, NV), 32, 0, s>>>(a, c0, c1, w, acc, 0);
+        seq_groups_kernel<PASS><<<dim3(ng, NV, 2), 32, 0, s>>>(a, c0, c1, w, acc, 1);
+    }
+    seq_walk_kernel<PASS><<<1, 32 * NV, 0, s>>>(a, c0, c1, w, acc);
     return cudaGetLastError();
 }
 
+// A slab's share of the sequential sums: the own planes, continuing acc.
 cudaError_t grav_moments_seq_slab(const GravArgs &a, int pass, double *acc, cudaStream_t s)
 {
-    const size_t sm = 9 * SEQ_CH * sizeof(double);
-    static std::atomic<unsigned long long> attr_set{0};
-    cudaError_t e = set_smem_once(attr_set, (const void *)moments_seq_slab_kernel, (int)sm);
-    if (e != cudaSuccess) return e;
-    moments_seq_slab_kernel<<<1, SEQ_NT, sm, s>>>(a, pass, acc);
-    return cudaGetLastError();
+    const long long sjk = (long long)a.g.ny * a.g.nz;
+    return pass == 0 ? seq_run<0>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s)
+                     : seq_run<1>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s);
+}
+
+cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s)
+{
+    if (a.g.n < SEQ_DIRECT) {
+        seq_direct_kernel<<<1, 288, 0, s>>>(a);
+        return cudaGetLastError();
+    }
+    if (a.scratch_len < 9) return cudaErrorInvalidValue;
+    for (int pass = 0; pass < 2; pass++) {
+        cudaError_t e = cudaMemsetAsync(a.scratch, 0, 9 * sizeof(double), s);
+        if (e == cudaSuccess)
+            e = pass == 0 ? seq_run<0>(a, 0, a.g.n, a.scratch, s) : seq_run<1>(a, 0, a.g.n, a.scratch, s);
+        if (e == cudaSuccess) e = grav_moments_seq_set(a, pass, a.scratch, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t grav_moments_seq_set(const GravArgs &a, int pass, const double *acc, cudaStream_t s)

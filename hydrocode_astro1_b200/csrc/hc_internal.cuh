@@ -178,12 +178,14 @@ struct GravArgs {
     DevScalars *sc;
     double *scratch;          // moment partial sums
     long long scratch_len;
+    void *seq;                // work of the sequential moments (grav_seq_bytes), or null
     double *mom;              // multipole results: 4 + ncoef
     double *gx, *gy, *gz;
 };
 
 // FP64 gravity (bit-exact) -- gravity_fp64.cu
 cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s);
+size_t grav_seq_bytes(const Geom &g);
 cudaError_t grav_moments_tree(const GravArgs &a, cudaStream_t s);
 // Moments of a slab (own planes [a.g.olo, a.g.ohi)).  Sequential order:
 // pass 0 / 1 continues the sums acc[0..4) / acc[0..9) (device memory) over
