@@ -94,6 +94,9 @@ struct hc_ctx {
     ResPlan rplan;
     void *exch;
     unsigned epoch;
+    // streaming passes (sor_stream.cuh) of grids that do not fit
+    int stream;                  // 0 not looked at yet, 1 in use, -1 the layout does not allow them
+    StreamTile tile[2];          // passes of 1 and of 2 iterations
     double *gx, *gy, *gz;
     double *res;
     int res_cap;
@@ -627,6 +630,59 @@ static bool resident_sweeps(hc_ctx *c, size_t elem)
     return c->resident == 1;
 }
 
+// Whether an FP32 context's sweeps run as streaming passes (where they do not
+// run resident).  FP64 keeps the separate sweeps: its windows hold half the
+// cells, and the passes measured 125 us an iteration at 256^3 against 112.
+static bool stream_sweeps(hc_ctx *c)
+{
+    if (c->cfg.sor_depth != 0 || c->cfg.precision != HC_FP32) return false;
+    if (c->stream == 0)
+        c->stream = mixed_stream_tile(c->g, 1, &c->tile[0]) && mixed_stream_tile(c->g, 2, &c->tile[1]) ? 1 : -1;
+    return c->stream == 1;
+}
+
+// The passes of a batch of iterations [it, end): two iterations each, a last
+// single one; buffer `cur` of the two holds the iterate.
+struct StreamRun {
+    int cur;     // buffer with the iterate before the batch
+    int pair;    // iterations of the last pass
+};
+template <typename F>
+static int stream_batch(hc_ctx *c, StreamRun &r, int it, int end, F pass)
+{
+    int b = r.cur;
+    for (int q = it; q < end;) {
+        const int its = end - q >= 2 ? 2 : 1;
+        const int rc = pass(its, b, q, r.pair, 0);
+        if (rc) return rc;
+        b ^= 1;
+        r.pair = its;
+        q += its;
+        c->launches += 1;
+        c->sor_launches += 1;
+    }
+    return HC_OK;
+}
+// The buffer that holds the iterate after the batch, of which `used`
+// iterations count (done) or all.  A pass of two whose first iteration ended
+// the solve is repeated with that one alone, from its input.
+template <typename F>
+static int stream_settle(hc_ctx *c, StreamRun &r, int it, int end, int used, F pass)
+{
+    const int n = used - it, full = n / 2;
+    const int b = r.cur ^ (full & 1);
+    r.cur = b;
+    if (n % 2) {
+        r.cur = b ^ 1;
+        if (used < end) {
+            c->launches += 1;
+            c->sor_launches += 1;
+            return pass(1, b, used - 1, 0, 1);
+        }
+    }
+    return HC_OK;
+}
+
 // Red-black SOR to tolerance, FP64 (gravity_solve_potential,
 // gravity_solver_3d.c:510-747).  Returns 0 / -1 like the reference, or a
 // negative HC_ERR_* code.
@@ -777,6 +833,7 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
     // passes of that many FP32 iterations per HBM pass on the natural layout
     const bool split = (c->cfg.sor_depth == 0 || c->cfg.sor_depth == -2 || c->cfg.sor_depth == -3) && c->g.nz >= 3;
     const bool resident = split && resident_sweeps(c, sizeof(float));
+    const bool stream = split && !resident && stream_sweeps(c);
     const bool wave2 = split && c->cfg.sor_depth == -2 && mixed_wave_split_ok(c->g);
     const int depth = wave2 ? 2 : (split ? -1 : c->cfg.sor_depth);
     int rc = ensure_res(c, a.max_iter);
@@ -890,6 +947,11 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
         // the passes write every interior cell of their output; its boundary
         // cells (zero for the correction) come from here
         if (wave2) CK(cudaMemsetAsync(c->e32b, 0, (size_t)split_len(c->g) * sizeof(float), c->s));
+        StreamRun run = { 0, 0 };
+        auto pass = [&](int its, int b, int q, int pair, int force) -> int {
+            CK(mixed_sor32_stream(a, c->tile[its - 1], its, eb[b], eb[b ^ 1], c->r32, q, pair, thresh, force, c->s));
+            return HC_OK;
+        };
         int it = 0, done = 0, last = 0, batch = 16, processed = 0, best_it = 0;
         double best = 1e300;
         if (!c->hslots && cudaMallocHost((void **)&c->hslots, 512 * sizeof(double)) != cudaSuccess)
@@ -903,6 +965,10 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
                                             c->s));
                     c->epoch += 4u * (unsigned)(end - it) + 16u;
                     c->sor_launches += 1;
+                } else if (stream) {
+                    rc = stream_batch(c, run, it, end, pass);
+                    if (rc) return rc;
+                    CK(mixed_stream_check(a, end, run.pair, thresh, c->s));
                 } else if (wave2) {
                     for (int q = it; q < end; q += 2) {
                         CK(mixed_sor32_split_pass(a, eb[(q / 2) & 1], eb[((q / 2) + 1) & 1], c->r32, q, thresh, c->s));
@@ -935,7 +1001,7 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
                     }
                     end = it + ((end - it + depth - 1) / depth) * depth;
                 }
-                if (!resident) CK(mixed_check(a, end, thresh, c->s));
+                if (!resident && !stream) CK(mixed_check(a, end, thresh, c->s));
                 c->launches += 1;
             }
             processed = end;
@@ -946,6 +1012,11 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
             if (rc) return rc;
             done = c->hsc->done;
             last = c->hsc->last_iter;
+            if (stream) {
+                FamTimer t(c, FAM_SOR);
+                rc = stream_settle(c, run, it, end, done ? last : end, pass);
+                if (rc) return rc;
+            }
             if (done || end >= budget) break;
             // stagnation guard: FP32 round-off floor reached before thresh
             for (int q = 0; q < nb; q++) {
@@ -962,7 +1033,8 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
         const int used = done ? last : processed;
         total += used;
         // the correction is in eb[passes % 2] for the blocked sweeps
-        const float *efinal = ((split && !wave2) || depth < 0) ? c->e32 : eb[(used / depth) & 1];
+        const float *efinal = stream ? eb[run.cur]
+                              : (split && !wave2) || depth < 0 ? c->e32 : eb[(used / depth) & 1];
         {
             FamTimer t(c, FAM_RES);
             CK(cudaMemsetAsync(&c->sc->resid_bits, 0, sizeof(unsigned long long), c->s));

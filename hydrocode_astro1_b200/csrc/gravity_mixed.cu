@@ -18,6 +18,7 @@
 #include "sor_resident.cuh"
 #include "sor_split.cuh"
 #include "sor_split_tma.cuh"
+#include "sor_stream.cuh"
 #include "sor_wave_split.cuh"
 #include "tmap.cuh"
 
@@ -801,6 +802,28 @@ cudaError_t mixed_sor32_resident(const GravArgs &a, float *e32, const float *r32
 {
     return run_resident<float>(p, e32, r32, make_split(a.g), sor_coef32(a), exch, epoch, a.res, it0, n, thresh, a.sc,
                                s);
+}
+
+bool mixed_stream_tile(const Geom &g, int its, StreamTile *out)
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return false;
+    return stream_tile(make_split(g), its, sms, out);
+}
+
+cudaError_t mixed_stream_check(const GravArgs &a, int iter0, int pair, double thresh, cudaStream_t s)
+{
+    stream_check_kernel<<<1, 1, 0, s>>>(a.res, iter0, pair, thresh, a.sc);
+    return cudaGetLastError();
+}
+
+cudaError_t mixed_sor32_stream(const GravArgs &a, const StreamTile &t, int its, const float *in, float *out,
+                               const float *r32, int iter0, int pair, double thresh, int force, cudaStream_t s)
+{
+    return run_stream(t, its, in, out, r32, make_split(a.g), sor_coef32(a), a.res, iter0, pair, thresh, force,
+                             a.sc, s);
 }
 
 cudaError_t mixed_sor32_split(const GravArgs &a, float *e32, const float *r32, int colour, int iter,

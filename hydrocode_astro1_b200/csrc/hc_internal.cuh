@@ -259,6 +259,20 @@ struct ResPlan {
     size_t smem = 0, exch_bytes = 0;
 };
 bool grav_resident_plan(const Geom &g, size_t elem, ResPlan *out);
+// FP32 passes of 1 or 2 iterations on larger grids (sor_stream.cuh), out of place:
+// windows of W rows x WV vectors
+struct StreamTile {
+    int W, WV;             // window: rows, vectors (16 bytes)
+    int BJ, BV;            // owned rows / vectors of a tile away from the grid's edges
+    int tj, tk, L, ch;     // tiles along j and k, planes of a chunk, chunks
+    unsigned magic;        // ceil(2^32 / WV), 0 for one
+};
+bool mixed_stream_tile(const Geom &g, int its, StreamTile *out);
+// iterations iter0 .. iter0 + its - 1 unless one of the `pair` before them
+// ended the solve (force: whatever they say); the check after the last pass
+cudaError_t mixed_sor32_stream(const GravArgs &a, const StreamTile &t, int its, const float *in, float *out,
+                               const float *r32, int iter0, int pair, double thresh, int force, cudaStream_t s);
+cudaError_t mixed_stream_check(const GravArgs &a, int iter0, int pair, double thresh, cudaStream_t s);
 cudaError_t grav_sor_resident(const GravArgs &a, double *phs, const double *rhs, const ResPlan &p, void *exch,
                               unsigned epoch, int it0, int n, cudaStream_t s);
 cudaError_t mixed_sor32_resident(const GravArgs &a, float *e32, const float *r32, const ResPlan &p, void *exch,
