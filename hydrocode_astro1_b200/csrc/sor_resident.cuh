@@ -319,6 +319,16 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     };
 
     if (*(volatile int *)&A.sc->done) return;
+    // iteration it0 - 1 (a sweep's, before the boundary values were set) may
+    // have been the last
+    if (A.it0 > 0 &&
+        __longlong_as_double(*reinterpret_cast<const volatile long long *>(A.res + A.it0 - 1)) < A.thresh) {
+        if (cta == 0 && tid == 0) {
+            A.sc->last_iter = A.it0;
+            A.sc->done = 1;
+        }
+        return;
+    }
     if (tid == 0) {
         quit = 0;
         bmax[0] = bmax[1] = 0;

@@ -33,7 +33,8 @@ def test_resident_fp64_capped(shape, max_iter):
     assert a[1:] == b[1:]
 
 
-@pytest.mark.parametrize("tol", [1e-2, 1e-3, 1e-5, 3e-7])
+# (1e3: the first iteration, which runs before the boundary values are set)
+@pytest.mark.parametrize("tol", [1e3, 1e-2, 1e-3, 1e-5, 3e-7])
 @pytest.mark.parametrize("shape", SHAPES[:7])
 def test_resident_fp64_stops_at_the_same_iteration(shape, tol):
     a, b = (solve64(shape, depth, 20000, tol) for depth in (0, -1))
