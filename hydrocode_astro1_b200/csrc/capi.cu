@@ -1275,17 +1275,6 @@ static HydroArgs hydro_args(hc_ctx *c)
     return a;
 }
 
-static int interior_chunks(const hc_ctx *c)
-{
-    long long tiles = (long long)((c->g.nz + 31) / 32) * ((c->g.ny + 7) / 8);
-    long long want = 148LL * 2 * 4;   // ~4 waves of 2 resident blocks per SM
-    long long ch = (want + tiles - 1) / tiles;
-    ch = std::max(1LL, std::min(ch, (long long)(c->g.nx - 2)));
-    // keep at least 8 planes per chunk so the prologue plane stays cheap
-    ch = std::min(ch, std::max(1LL, (long long)(c->g.nx - 2) / 8));
-    return (int)ch;
-}
-
 // One godunov step on the device state (no host synchronisation).
 static int step_once(hc_ctx *c, int *grav_status)
 {
@@ -1320,24 +1309,13 @@ static int step_once(hc_ctx *c, int *grav_status)
             CK(fp64_plm_interior(a, c->plm, c->s));
             c->launches += 1;
         } else {
-            CK(f64 ? fp64_interior(a, interior_chunks(c), c->s) : fp32_interior(a, interior_chunks(c), c->s));
+            CK(f64 ? fp64_interior(a, c->s) : fp32_interior(a, c->s));
         }
     }
     {
         FamTimer t(c, FAM_BC);
-        CK(f64 ? fp64_boundary_source(a, c->s) : fp32_boundary_source(a, c->s));
-        c->launches += 3;
-        for (int ax = 0; ax < 3; ax++)
-            if (c->cfg.bc[2 * ax] == 0 && c->cfg.bc[2 * ax + 1] == 0) {
-                CK(f64 ? fp64_periodic(a, ax, c->s) : fp32_periodic(a, ax, c->s));
-                c->launches++;
-            }
-        for (int ax = 0; ax < 3; ax++) {
-            CK(f64 ? fp64_bc(a, ax, c->s) : fp32_bc(a, ax, c->s));
-            c->launches++;
-        }
-        CK(f64 ? fp64_cfl_boundary(a, c->s) : fp32_cfl_boundary(a, c->s));
-        c->launches++;
+        CK(f64 ? fp64_boundary(a, c->s) : fp32_boundary(a, c->s));
+        c->launches += 3;   // with dt and the interior
     }
     c->hydro_launches++;
     c->cur ^= 1;

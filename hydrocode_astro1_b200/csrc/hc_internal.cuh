@@ -123,11 +123,8 @@ struct HydroArgs {
 // FP64 (bit-exact) hydro path -- hydro_fp64.cu
 cudaError_t fp64_cfl_full(const HydroArgs &a, cudaStream_t s);
 cudaError_t fp64_dt(const HydroArgs &a, cudaStream_t s);
-cudaError_t fp64_interior(const HydroArgs &a, int chunks, cudaStream_t s);
-cudaError_t fp64_boundary_source(const HydroArgs &a, cudaStream_t s);
-cudaError_t fp64_periodic(const HydroArgs &a, int axis, cudaStream_t s);
-cudaError_t fp64_bc(const HydroArgs &a, int axis, cudaStream_t s);
-cudaError_t fp64_cfl_boundary(const HydroArgs &a, cudaStream_t s);
+cudaError_t fp64_interior(const HydroArgs &a, cudaStream_t s);
+cudaError_t fp64_boundary(const HydroArgs &a, cudaStream_t s);
 cudaError_t fp64_aos_to_soa(const double *aos, double *const q[5], long long n, cudaStream_t s);
 cudaError_t fp64_soa_to_aos(const double *const q[5], double *aos, long long n, cudaStream_t s);
 // profile-based initial state on the device -- ics_device.cu
@@ -151,11 +148,8 @@ cudaError_t cons_sums(const ConsFields<T> &q, long long n, double *partial, doub
 // FP32 hydro path -- hydro_fp32.cu
 cudaError_t fp32_cfl_full(const HydroArgs &a, cudaStream_t s);
 cudaError_t fp32_dt(const HydroArgs &a, cudaStream_t s);
-cudaError_t fp32_interior(const HydroArgs &a, int chunks, cudaStream_t s);
-cudaError_t fp32_boundary_source(const HydroArgs &a, cudaStream_t s);
-cudaError_t fp32_periodic(const HydroArgs &a, int axis, cudaStream_t s);
-cudaError_t fp32_bc(const HydroArgs &a, int axis, cudaStream_t s);
-cudaError_t fp32_cfl_boundary(const HydroArgs &a, cudaStream_t s);
+cudaError_t fp32_interior(const HydroArgs &a, cudaStream_t s);
+cudaError_t fp32_boundary(const HydroArgs &a, cudaStream_t s);
 cudaError_t fp32_from_fp64(const double *const q64[5], float *const q32[5], long long n, cudaStream_t s);
 cudaError_t fp32_to_fp64(const float *const q32[5], double *const q64[5], long long n, cudaStream_t s);
 cudaError_t f32_to_f64(const float *a, double *b, long long n, cudaStream_t s);

@@ -156,7 +156,7 @@ static cudaError_t pk_interior(const HydroArgs &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t fp32_interior(const HydroArgs &a, int chunks, cudaStream_t s)
+cudaError_t fp32_interior(const HydroArgs &a, cudaStream_t s)
 {
     if (hydro32_choice() == 0 && tma_usable(a)) {
         cudaError_t e = pk_interior(a, s);
@@ -178,52 +178,13 @@ cudaError_t fp32_interior(const HydroArgs &a, int chunks, cudaStream_t s)
             return cudaGetLastError();
         }
     }
-    constexpr size_t sm = interior_smem<float, TK, TJ>();
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(interior_kernel<float, TK, TJ>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
-    int nint = a.g.nx - 2;
-    int ilen = (nint + chunks - 1) / chunks;
-    chunks = (nint + ilen - 1) / ilen;
-    dim3 grid((a.g.nz + TK - 1) / TK, (a.g.ny + TJ - 1) / TJ, chunks);
-    interior_kernel<float, TK, TJ><<<grid, dim3(TK, TJ), sm, s>>>(a, ilen);
-    return cudaGetLastError();
+    return launch_interior<float, TK, TJ>(a, s);
 }
 
-cudaError_t fp32_boundary_source(const HydroArgs &a, cudaStream_t s)
+cudaError_t fp32_boundary(const HydroArgs &a, cudaStream_t s)
 {
-    long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
-    boundary_source_kernel<float><<<grid_for(nb, 256), 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-static long long face_count(const HydroArgs &a, int axis)
-{
-    const int n[3] = { a.g.nx, a.g.ny, a.g.nz };
-    return (long long)((axis == 0) ? n[1] : n[0]) * ((axis == 2) ? n[1] : n[2]);
-}
-
-cudaError_t fp32_periodic(const HydroArgs &a, int axis, cudaStream_t s)
-{
-    periodic_kernel<float><<<grid_for(face_count(a, axis), 256), 256, 0, s>>>(a, axis);
-    return cudaGetLastError();
-}
-
-cudaError_t fp32_bc(const HydroArgs &a, int axis, cudaStream_t s)
-{
-    bc_kernel<float><<<grid_for(face_count(a, axis), 256), 256, 0, s>>>(a, axis);
-    return cudaGetLastError();
-}
-
-cudaError_t fp32_cfl_boundary(const HydroArgs &a, cudaStream_t s)
-{
-    long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
-    int blocks = (int)std::min<long long>(grid_for(nb, 256), 148 * 4);
-    cfl_boundary_kernel<float><<<blocks, 256, 0, s>>>(a);
+    const long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
+    boundary_kernel<float><<<grid_for(nb, 256), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

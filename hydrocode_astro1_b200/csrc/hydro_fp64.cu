@@ -45,50 +45,12 @@ cudaError_t fp64_dt(const HydroArgs &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t fp64_interior(const HydroArgs &a, int chunks, cudaStream_t s)
-{
-    constexpr size_t sm = interior_smem<double, TK, TJ>();
-    static std::atomic<unsigned long long> attr_set{0};
-    cudaError_t e = set_smem_once(attr_set, (const void *)interior_kernel<double, TK, TJ>, (int)sm);
-    if (e != cudaSuccess) return e;
-    int nint = a.g.nx - 2;
-    int ilen = (nint + chunks - 1) / chunks;
-    chunks = (nint + ilen - 1) / ilen;
-    dim3 grid((a.g.nz + TK - 1) / TK, (a.g.ny + TJ - 1) / TJ, chunks);
-    interior_kernel<double, TK, TJ><<<grid, dim3(TK, TJ), sm, s>>>(a, ilen);
-    return cudaGetLastError();
-}
+cudaError_t fp64_interior(const HydroArgs &a, cudaStream_t s) { return launch_interior<double, TK, TJ>(a, s); }
 
-cudaError_t fp64_boundary_source(const HydroArgs &a, cudaStream_t s)
+cudaError_t fp64_boundary(const HydroArgs &a, cudaStream_t s)
 {
-    long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
-    boundary_source_kernel<double><<<grid_for(nb, 256), 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-static long long face_count(const HydroArgs &a, int axis)
-{
-    const int n[3] = { a.g.nx, a.g.ny, a.g.nz };
-    return (long long)((axis == 0) ? n[1] : n[0]) * ((axis == 2) ? n[1] : n[2]);
-}
-
-cudaError_t fp64_periodic(const HydroArgs &a, int axis, cudaStream_t s)
-{
-    periodic_kernel<double><<<grid_for(face_count(a, axis), 256), 256, 0, s>>>(a, axis);
-    return cudaGetLastError();
-}
-
-cudaError_t fp64_bc(const HydroArgs &a, int axis, cudaStream_t s)
-{
-    bc_kernel<double><<<grid_for(face_count(a, axis), 256), 256, 0, s>>>(a, axis);
-    return cudaGetLastError();
-}
-
-cudaError_t fp64_cfl_boundary(const HydroArgs &a, cudaStream_t s)
-{
-    long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
-    int blocks = (int)std::min<long long>(grid_for(nb, 256), 148 * 4);
-    cfl_boundary_kernel<double><<<blocks, 256, 0, s>>>(a);
+    const long long nb = boundary_count(a.g.nx, a.g.ny, a.g.nz, true);
+    boundary_kernel<double><<<grid_for(nb, 256), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -10,15 +10,18 @@
 //                      shared through shared memory, flux difference update
 //                      (:729-764), floors (:765-768), gravity source (:597-631)
 //                      with g = -grad(phi) formed in place, next-step CFL max
-//   boundary source    the gravity source on the six faces (never flux-updated,
-//                      :729-731) with g copied from the nearest interior cell
-//                      (gravity_solver_3d.c:842-897)
-//   periodic / bc      hydro_solver_3d.c:779-807 then :456-552, axis by axis
-//   boundary CFL       max signal speed of the final face cells
+//   boundary kernel    the six faces (never flux-updated, :729-731): gravity
+//                      source with g copied from the nearest interior cell
+//                      (gravity_solver_3d.c:842-897), periodic copies and
+//                      boundary conditions (hydro_solver_3d.c:779-807 then
+//                      :456-552, axis by axis), max signal speed
 // The state is double-buffered: every kernel reads step-n values and writes
 // the step-(n+1) buffer, which is what the reference's separate flux arrays
 // give it.
 #pragma once
+#include <algorithm>
+#include <atomic>
+
 #include "hc_internal.cuh"
 #include "hc_math.cuh"
 
@@ -82,7 +85,7 @@ __device__ __forceinline__ CellS<T> make_cell(const Cons<T> &q, T gm1, T gam)
 // --------------------------------------------------------------------------
 template <typename T, int TK, int TJ>
 __global__ void __launch_bounds__(TK * TJ)
-interior_kernel(HydroArgs a, int ilen)
+interior_kernel(HydroArgs a, int ilen, int k00, int j00)   // k00, j00: first cell of the tiles
 {
     constexpr int SK = TK + 2, SJ = TJ + 2, NS = SK * SJ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -94,7 +97,7 @@ interior_kernel(HydroArgs a, int ilen)
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
     const long long sI = (long long)ny * nz, sJ = nz;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TK + tx;
-    const int k0 = blockIdx.x * TK, j0 = blockIdx.y * TJ;
+    const int k0 = k00 + blockIdx.x * TK, j0 = j00 + blockIdx.y * TJ;
     const int k = k0 + tx, j = j0 + ty;
     const int ib = 1 + blockIdx.z * ilen;
     const int ie = min(nx - 1, ib + ilen);   // exclusive; interior is [1, nx-2]
@@ -208,6 +211,58 @@ constexpr size_t interior_smem()
            sizeof(Cons<T>) * ((TJ + 1) * TK + TJ * (TK + 1));
 }
 
+// Planes of a chunk along i: the fewest waves x (planes + the prologue's one)
+// over the CTAs that run at once.  (A fixed four waves of at least 8 planes
+// left most SMs idle on small grids.  FP64, before -> now: 16^3 107 -> 19 us,
+// 64^3 66 -> 40, 128^3 246 -> 220, 256^3 1664 -> 1550.)
+inline int chunk_planes(long long tiles, int nint, long long slots)
+{
+    int best = nint;
+    long long cost = -1;
+    for (int l = 1; l <= nint; l++) {
+        const long long ctas = tiles * ((nint + l - 1) / l), c = (ctas + slots - 1) / slots * (l + 1);
+        if (cost < 0 || c <= cost) {
+            cost = c;
+            best = l;
+        }
+    }
+    return best;
+}
+
+// One launch of interior_kernel.
+template <typename T, int TK, int TJ>
+cudaError_t launch_interior(const HydroArgs &a, cudaStream_t s)
+{
+    constexpr size_t sm = interior_smem<T, TK, TJ>();
+    static std::atomic<unsigned long long> attr_set{0};
+    cudaError_t e = set_smem_once(attr_set, (const void *)interior_kernel<T, TK, TJ>, (int)sm);
+    if (e != cudaSuccess) return e;
+    static std::atomic<int> slots_dev[64];
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int slots = (dev >= 0 && dev < 64) ? slots_dev[dev].load() : 0;
+    if (!slots) {
+        int per_sm = 0, sms = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, interior_kernel<T, TK, TJ>, TK * TJ, sm);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        slots = std::max(1, per_sm) * sms;
+        if (dev >= 0 && dev < 64) slots_dev[dev].store(slots);
+    }
+    // tiles from cell 0 (aligned rows) or, where that saves a tile, from the
+    // first interior cell (101 x 99 x 97 FP64: 146 -> 117 us)
+    auto tiles = [](int n, int t, int &o) {
+        o = (n - 2 + t - 1) / t < (n - 1 + t - 1) / t ? 1 : 0;
+        return (n - 1 - o + t - 1) / t;
+    };
+    int k00, j00;
+    const int tk = tiles(a.g.nz, TK, k00), tj = tiles(a.g.ny, TJ, j00), nint = a.g.nx - 2;
+    const int ilen = chunk_planes((long long)tk * tj, nint, slots);
+    interior_kernel<T, TK, TJ><<<dim3(tk, tj, (nint + ilen - 1) / ilen), dim3(TK, TJ), sm, s>>>(a, ilen, k00, j00);
+    return cudaGetLastError();
+}
+
 // --------------------------------------------------------------------------
 // small kernels
 // --------------------------------------------------------------------------
@@ -239,97 +294,80 @@ __global__ void cfl_full_kernel(HydroArgs a)
                  reinterpret_cast<unsigned int *>(&a.sc->smax[a.step_parity]));
 }
 
+// The face cells, in one launch: gravity source, periodic copies, boundary
+// conditions and their signal speed.  The reference applies these one after
+// the other to whole faces (source :612-628, periodic x, y, z :779-807, then
+// conditions x, y, z :456-552); each step either leaves a cell, copies the
+// value another cell has before it, or flips the cell's own velocity.  So a
+// cell's final value is one cell's value after the source -- found by walking
+// the steps backwards -- with the flips on the way applied in order; nothing
+// is read that this launch writes.  (One launch per step read and wrote the
+// faces up to six times, the z faces a sector per cell.  With the dt kernel, per
+// step: 256^3 FP32 109 -> 46 us, 16^3 FP64 35 -> 17 us.)
 template <typename T>
-__global__ void boundary_source_kernel(HydroArgs a)
-{
-    const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
-    const long long nb = boundary_count(nx, ny, nz, true);
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= nb) return;
-    int i, j, k;
-    boundary_cell(t, nx, ny, nz, true, i, j, k);
-    const long long sI = (long long)ny * nz, sJ = nz;
-    const long long c = i * sI + j * sJ + k;
-    const T *const *qin = reinterpret_cast<const T *const *>(a.qin);
-    T *const *qout = reinterpret_cast<T *const *>(a.qout);
-    Cons<T> q = ld_cons(qin, c);
-    if (a.gravity) {
-        // g on a boundary cell equals g of the nearest interior cell after the
-        // x, y, z copy passes of gravity_compute_acceleration (:842-897)
-        int ci = min(max(i, 1), nx - 2), cj = min(max(j, 1), ny - 2), ck = min(max(k, 1), nz - 2);
-        long long cc = ci * sI + cj * sJ + ck;
-        const double *ph = a.phig;
-        double ax = -(ph[cc + sI] - ph[cc - sI]) / (2.0 * a.g.dx);
-        double ay = -(ph[cc + sJ] - ph[cc - sJ]) / (2.0 * a.g.dy);
-        double az = -(ph[cc + 1] - ph[cc - 1]) / (2.0 * a.g.dz);
-        gravity_source(q, ax, ay, az, (T)a.sc->dt);
-    }
-    st_cons(qout, c, q);
-}
-
-// index of (u,v) on the face plane normal to `axis`
-__device__ __forceinline__ long long face_index(int axis, int side_idx, int u, int v, int ny, int nz)
-{
-    const long long sI = (long long)ny * nz, sJ = nz;
-    if (axis == 0) return side_idx * sI + u * sJ + v;
-    if (axis == 1) return u * sI + side_idx * sJ + v;
-    return u * sI + v * sJ + side_idx;
-}
-
-template <typename T>
-__global__ void periodic_kernel(HydroArgs a, int axis)
+__device__ __forceinline__ Cons<T> boundary_value(const HydroArgs &a, int i, int j, int k)
 {
     const int n[3] = { a.g.nx, a.g.ny, a.g.nz };
-    const int nu = (axis == 0) ? n[1] : n[0], nv = (axis == 2) ? n[1] : n[2];
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)nu * nv) return;
-    const int u = (int)(t / nv), v = (int)(t % nv);
-    T *const *q = reinterpret_cast<T *const *>(a.qout);
-    long long c0 = face_index(axis, 0, u, v, n[1], n[2]);
-    long long c1 = face_index(axis, n[axis] - 1, u, v, n[1], n[2]);
-    Cons<T> s = ld_cons(reinterpret_cast<const T *const *>(a.qout), c1);
-    st_cons(q, c0, s);
-}
-
-template <typename T>
-__global__ void bc_kernel(HydroArgs a, int axis)
-{
-    const int n[3] = { a.g.nx, a.g.ny, a.g.nz };
-    const int nu = (axis == 0) ? n[1] : n[0], nv = (axis == 2) ? n[1] : n[2];
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)nu * nv) return;
-    const int u = (int)(t / nv), v = (int)(t % nv);
-    T *const *q = reinterpret_cast<T *const *>(a.qout);
-    const T *const *qc = reinterpret_cast<const T *const *>(a.qout);
     const T gm1 = (T)(a.gamma - 1.0);
-    for (int side = 0; side < 2; side++) {
-        int type = a.bc[2 * axis + side];
-        int ib = side ? n[axis] - 1 : 0, in = side ? n[axis] - 2 : 1;
-        long long cb = face_index(axis, ib, u, v, n[1], n[2]);
-        if (type == 1) {            // BC_REFLECTIVE: negate own normal velocity
-            Prim<T> w = to_prim(ld_cons(qc, cb), gm1);
-            w.v[axis] = -w.v[axis];
-            st_cons(q, cb, to_cons(w, gm1));
-        } else if (type == 2) {     // BC_OUTFLOW: copy the neighbour
-            st_cons(q, cb, ld_cons(qc, face_index(axis, in, u, v, n[1], n[2])));
-        }
+    int x[3] = { i, j, k };
+    bool flip[3] = { false, false, false };
+#pragma unroll
+    for (int ax = 2; ax >= 0; ax--) {
+        const bool lo = x[ax] == 0, hi = x[ax] == n[ax] - 1;
+        if (!lo && !hi) continue;
+        const int type = a.bc[2 * ax + (hi ? 1 : 0)];
+        if (type == 2) x[ax] = hi ? n[ax] - 2 : 1;   // BC_OUTFLOW: the neighbour
+        else if (type == 1) flip[ax] = true;         // BC_REFLECTIVE: negate own normal velocity
     }
+#pragma unroll
+    for (int ax = 2; ax >= 0; ax--)
+        if (x[ax] == 0 && a.bc[2 * ax] == 0 && a.bc[2 * ax + 1] == 0) x[ax] = n[ax] - 1;   // periodic
+    const long long sI = (long long)n[1] * n[2], sJ = n[2];
+    const long long c = x[0] * sI + x[1] * sJ + x[2];
+    bool face = false;
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) face = face || x[ax] == 0 || x[ax] == n[ax] - 1;
+    Cons<T> q;
+    if (face) {
+        q = ld_cons(reinterpret_cast<const T *const *>(a.qin), c);
+        if (a.gravity) {
+            // g on a boundary cell equals g of the nearest interior cell after the
+            // x, y, z copy passes of gravity_compute_acceleration (:842-897)
+            const int ci = min(max(x[0], 1), n[0] - 2), cj = min(max(x[1], 1), n[1] - 2), ck = min(max(x[2], 1), n[2] - 2);
+            const long long cc = ci * sI + cj * sJ + ck;
+            const double *ph = a.phig;
+            double ax = -(ph[cc + sI] - ph[cc - sI]) / (2.0 * a.g.dx);
+            double ay = -(ph[cc + sJ] - ph[cc - sJ]) / (2.0 * a.g.dy);
+            double az = -(ph[cc + 1] - ph[cc - 1]) / (2.0 * a.g.dz);
+            gravity_source(q, ax, ay, az, (T)a.sc->dt);
+        }
+    } else {
+        q = ld_cons(reinterpret_cast<const T *const *>(a.qout), c);
+    }
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++)
+        if (flip[ax]) {
+            Prim<T> w = to_prim(q, gm1);
+            w.v[ax] = -w.v[ax];
+            q = to_cons(w, gm1);
+        }
+    return q;
 }
 
 template <typename T>
-__global__ void cfl_boundary_kernel(HydroArgs a)
+__global__ void __launch_bounds__(256) boundary_kernel(HydroArgs a)
 {
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
     const long long nb = boundary_count(nx, ny, nz, true);
+    const long long t = blockIdx.x * 256LL + threadIdx.x;
     const T gam = (T)a.gamma, gm1 = (T)(a.gamma - 1.0);
-    const T *const *q = reinterpret_cast<const T *const *>(a.qout);
     T m = (T)0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nb;
-         t += (long long)gridDim.x * blockDim.x) {
+    if (t < nb) {
         int i, j, k;
         boundary_cell(t, nx, ny, nz, true, i, j, k);
-        long long c = ((long long)i * ny + j) * nz + k;
-        m = tmax(m, signal_speed(to_prim(ld_cons(q, c), gm1), gam));
+        const Cons<T> q = boundary_value<T>(a, i, j, k);
+        st_cons(reinterpret_cast<T *const *>(a.qout), ((long long)i * ny + j) * nz + k, q);
+        m = signal_speed(to_prim(q, gm1), gam);
     }
     block_max_to(m, &a.sc->smax[a.step_parity ^ 1],
                  reinterpret_cast<unsigned int *>(&a.sc->smax[a.step_parity ^ 1]));
