@@ -48,7 +48,13 @@ __device__ __forceinline__ void prim_arr(const Prim<double> &w, double *o)
     o[4] = w.p;
 }
 
-__global__ void __launch_bounds__(256) plm_predict_kernel(HydroArgs a, double *__restrict__ pl)
+// Both kernels wait on chains of FP64 divisions: at 156 to 179 registers one
+// block of 256 threads fitted an SM and the FP64 pipe was busy 20 to 29% of the
+// time.  Five or six blocks of 128 (96 and 80 registers, a few spills) keep
+// 20 to 24 warps in flight: 128^3 928 -> 545 us, 64^3 124 -> 79.
+constexpr int PLM_NT = 128;
+
+__global__ void __launch_bounds__(PLM_NT, 6) plm_predict_kernel(HydroArgs a, double *__restrict__ pl)
 {
     const Geom g = a.g;
     const long long n = g.n, sI = (long long)g.ny * g.nz, sJ = g.nz;
@@ -131,7 +137,7 @@ __device__ __forceinline__ Cons<double> plm_flux(const double *__restrict__ pl, 
     return hllc<A>(qL, wL, csound(wL, gam), qR, wR, csound(wR, gam));
 }
 
-__global__ void __launch_bounds__(256) plm_update_kernel(HydroArgs a, const double *__restrict__ pl)
+__global__ void __launch_bounds__(PLM_NT, 5) plm_update_kernel(HydroArgs a, const double *__restrict__ pl)
 {
     const Geom g = a.g;
     const long long n = g.n, sI = (long long)g.ny * g.nz, sJ = g.nz;
@@ -186,10 +192,10 @@ cudaError_t fp64_plm_interior(const HydroArgs &a, double *pl, cudaStream_t s)
 {
     if (a.g.nx < 3 || a.g.ny < 3 || a.g.nz < 3) return cudaErrorInvalidValue;
     const long long n = a.g.n, nint = (long long)(a.g.nx - 2) * (a.g.ny - 2) * (a.g.nz - 2);
-    const int b1 = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
-    const int b2 = (int)std::min<long long>((nint + 255) / 256, 148LL * 16);
-    plm_predict_kernel<<<b1, 256, 0, s>>>(a, pl);
-    plm_update_kernel<<<b2, 256, 0, s>>>(a, pl);
+    const int b1 = (int)std::min<long long>((n + PLM_NT - 1) / PLM_NT, 148LL * 32);
+    const int b2 = (int)std::min<long long>((nint + PLM_NT - 1) / PLM_NT, 148LL * 32);
+    plm_predict_kernel<<<b1, PLM_NT, 0, s>>>(a, pl);
+    plm_update_kernel<<<b2, PLM_NT, 0, s>>>(a, pl);
     return cudaGetLastError();
 }
 
