@@ -189,21 +189,75 @@ conv3_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
 // ---------------------------------------------------------------- weight gradient
 constexpr int WG_NT = 256;
 constexpr int WG_MT = 4;                   // 128-row tiles: taps 0-7, 8-15, 16-23, 24-26
+constexpr int WG_ST = 3;                   // chunks staged in shared memory
 struct WgradSmem {
-    __align__(128) unsigned char a[2][WG_MT][TM * KC * 2];   // 2 x 4 x 16 KB
-    __align__(128) unsigned char b[2][CH * KC * 2];          // 2 x 2 KB
-    __align__(8) uint64_t bar[2];
+    __align__(128) unsigned char a[WG_ST][WG_MT][TM * KC * 2];   // 3 x 4 x 16 KB
+    __align__(128) unsigned char b[WG_ST][CH * KC * 2];          // 3 x 2 KB
+    __align__(8) uint64_t bar[WG_ST];
     uint32_t tmem;
 };
 
 // byte offset of (mn, k) in an MN-major no-swizzle tile with KC columns:
 // 8 consecutive mn = one 16-byte row, 8 rows (k) per core matrix
-__host__ __device__ __forceinline__ uint32_t mnmajor_off(int mn, int k, int kc)
+__host__ __device__ __forceinline__ constexpr uint32_t mnmajor_off(int mn, int k, int kc)
 {
     return (uint32_t)((mn >> 3) * (16 * kc) + (k >> 3) * 128 + (k & 7) * 16 + (mn & 7) * 2);
 }
 
-// partial[cta][tap][ci][co] over the CTA's voxel chunks [c0, c1)
+// 16 bytes to shared memory without passing registers; zeros if !in
+__device__ __forceinline__ void cp16(unsigned char *dst, const __nv_bfloat16 *src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(in ? 16 : 0)
+                 : "memory");
+}
+
+// Taps G, G+2, ... of one voxel and channel half into the A tiles of a stage;
+// the warps of G = 1 have one tap less and fetch dY instead.
+template <int G>
+__device__ __forceinline__ void wgrad_fetch(WgradSmem &sm, int st, const __nv_bfloat16 *__restrict__ x,
+                                            const __nv_bfloat16 *__restrict__ dy, const Dims &d, long long v, int kk,
+                                            int half)
+{
+    const bool live = v < d.n;
+    int i = 0, j = 0, k = 0;
+    if (d.n <= 0x7fffffffLL) {
+        const unsigned u = (unsigned)v, row = u / (unsigned)d.nz;   // (the divisions of the 64-bit form cost 5x)
+        k = (int)(u - row * (unsigned)d.nz);
+        i = (int)(row / (unsigned)d.ny);
+        j = (int)(row - (unsigned)i * (unsigned)d.ny);
+    } else {
+        voxel_ijk(d, v, i, j, k);
+    }
+    const bool ok_i[3] = { live && i > 0, live, live && i < d.nx - 1 };
+    const bool ok_j[3] = { j > 0, true, j < d.ny - 1 };
+    const bool ok_k[3] = { k > 0, true, k < d.nz - 1 };
+    const long long plane = (long long)d.ny * d.nz;
+    const __nv_bfloat16 *xh = x + half * 8;
+    unsigned char *dst = sm.a[st][0] + mnmajor_off(half * 8, kk, KC);
+#pragma unroll
+    for (int m = 0; m < 14; m++) {
+        constexpr int STEP = mnmajor_off(CH, 0, KC), TILE = TM * KC * 2;
+        const int tap = G + 2 * m;
+        if (tap < NTAP) {
+            const int a = tap / 9, b = (tap / 3) % 3, c = tap % 3;
+            const bool in = ok_i[a] && ok_j[b] && ok_k[c];
+            const long long nb = v + (a - 1) * plane + (b - 1) * d.nz + (c - 1);
+            cp16(dst + (tap >> 3) * TILE + (tap & 7) * STEP, in ? xh + nb * CH : x, in);
+        }
+    }
+    if (G == 1) cp16(sm.b[st] + mnmajor_off(half * 8, kk, KC), live ? dy + v * CH + half * 8 : dy, live);
+}
+
+// partial[cta][tap][ci][co] over the CTA's voxel chunks [c0, c1).
+//
+// Each chunk of 64 voxels is staged as the 27 shifted copies of its x (the A
+// operand of 16 MMAs of 16 voxels), and what bounds it is shared memory: 54 KB
+// written and 72 KB read by the MMAs per chunk, about 1000 cycles.  Chunks are
+// fetched by cp.async two ahead of the one the tensor core works on; a warp
+// takes 16 voxels x 2 halves, 512 contiguous bytes.  Rows of taps past 26 are
+// never written and never read back.  128^3 voxels 1650 -> 261 us, 64^3 205 ->
+// 37 us against fetching through registers one chunk at a time, with a 64-bit
+// division chain per 16 bytes.
 __global__ void __launch_bounds__(WG_NT)
 wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy, float *__restrict__ partial,
              Dims d, int chunks_per_cta, int *err)
@@ -213,84 +267,68 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long nchunk = (d.n + KC - 1) / KC;
     const long long c0 = (long long)blockIdx.x * chunks_per_cta;
-    const long long c1 = min(nchunk, c0 + chunks_per_cta);
+    const int nq = (int)(min(nchunk, c0 + chunks_per_cta) - c0);
+    const int kk = (warp & 3) * 16 + (lane >> 4) * 8 + (lane & 7), half = (lane >> 3) & 1;
 
     if (warp == 0) {
         tc::tmem_alloc(&sm.tmem, 64);
         tc::fence_before();
     }
-    if (tid == 0) {
-        tc::bar_init(&sm.bar[0], 1);
-        tc::bar_init(&sm.bar[1], 1);
-    }
+    if (tid == 0)
+        for (int q = 0; q < WG_ST; q++) tc::bar_init(&sm.bar[q], 1);
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = sm.tmem;
     constexpr uint32_t IDESC = tc::idesc_bf16(TM, CH) | (1u << 15) | (1u << 16);
     bool ok = true;
-    int issued = 0;
 
-    for (long long c = c0; c < c1; c++) {
-        const int q = (int)(c - c0), buf = q & 1;
-        if (q >= 2) ok = tc::bar_wait(&sm.bar[buf], ((q - 2) >> 1) & 1) && ok;
-        // A: 4 tiles x (8 taps x 2 halves) x 64 voxels of 16-byte rows; B: 2 halves x 64
-        for (int t = tid; t < KC * (32 * 2 + 2); t += WG_NT) {
-            const int kk = t % KC, slot = t / KC;      // slot 0..63: (tap 0..31, half); 64..65: dy halves
-            const long long v = c * KC + kk;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (slot < 64) {
-                const int tap = slot >> 1, half = slot & 1;
-                if (v < d.n && tap < NTAP) {
-                    int i, j, k;
-                    voxel_ijk(d, v, i, j, k);
-                    const long long nb = neighbour(d, i, j, k, tap);
-                    if (nb >= 0) val = *reinterpret_cast<const uint4 *>(x + nb * CH + half * 8);
-                }
-                const int tile = tap >> 3, row = (tap & 7) * 16 + half * 8;
-                *reinterpret_cast<uint4 *>(sm.a[buf][tile] + mnmajor_off(row, kk, KC)) = val;
-            } else {
-                const int half = slot - 64;
-                if (v < d.n) val = *reinterpret_cast<const uint4 *>(dy + v * CH + half * 8);
-                *reinterpret_cast<uint4 *>(sm.b[buf] + mnmajor_off(half * 8, kk, KC)) = val;
-            }
-        }
-        tc::fence_smem_to_async();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after();
-            const uint32_t sb = tc::smem_u32(sm.b[buf]);
+    for (int q = -2; q < nq; q++) {   // q < 0: the first two fetches
+        if (q >= 0) {
+            const int st = q % WG_ST;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");   // all but the chunk after this one
+            tc::fence_smem_to_async();
+            __syncthreads();
+            if (tid == 0) {
+                tc::fence_after();
+                const uint32_t sb = tc::smem_u32(sm.b[st]);
 #pragma unroll
-            for (int tile = 0; tile < WG_MT; tile++) {
-                const uint32_t sa = tc::smem_u32(sm.a[buf][tile]);
+                for (int tile = 0; tile < WG_MT; tile++) {
+                    const uint32_t sa = tc::smem_u32(sm.a[st][tile]);
 #pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    const uint64_t da = tc::sdesc(sa + s * 256, 128, 16 * KC);
-                    const uint64_t db = tc::sdesc(sb + s * 256, 128, 16 * KC);
-                    tc::mma_bf16(tmem + tile * 16, da, db, IDESC, (q > 0 || s > 0) ? 1u : 0u);
+                    for (int s = 0; s < 4; s++) {
+                        const uint64_t da = tc::sdesc(sa + s * 256, 128, 16 * KC);
+                        const uint64_t db = tc::sdesc(sb + s * 256, 128, 16 * KC);
+                        tc::mma_bf16(tmem + tile * 16, da, db, IDESC, (q > 0 || s > 0) ? 1u : 0u);
+                    }
                 }
+                tc::mma_commit(&sm.bar[st]);
             }
-            tc::mma_commit(&sm.bar[buf]);
+            // the stage of chunk q + 2 is that of q - 1
+            if (q >= 1) ok = tc::bar_wait(&sm.bar[(q - 1) % WG_ST], ((q - 1) / WG_ST) & 1) && ok;
         }
-        issued = q + 1;
+        if (q + 2 < nq) {
+            const long long v = (c0 + q + 2) * KC + kk;
+            if (warp < 4) wgrad_fetch<0>(sm, (q + 2) % WG_ST, x, dy, d, v, kk, half);
+            else wgrad_fetch<1>(sm, (q + 2) % WG_ST, x, dy, d, v, kk, half);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
     float *p = partial + (size_t)blockIdx.x * (WG_MT * TM * CH);
-    if (issued > 0) {
-        const int ql = issued - 1;
-        ok = tc::bar_wait(&sm.bar[ql & 1], (ql >> 1) & 1) && ok;   // the last commit covers all
-        if (ql >= 1) ok = tc::bar_wait(&sm.bar[(ql - 1) & 1], ((ql - 1) >> 1) & 1) && ok;
-        tc::fence_after();
+    ok = tc::bar_wait(&sm.bar[(nq - 1) % WG_ST], ((nq - 1) / WG_ST) & 1) && ok;   // the last commit covers all
+    tc::fence_after();
 #pragma unroll
-        for (int tile = 0; tile < WG_MT; tile++) {
-            if (warp < 4) {   // warps 0-3 own TMEM lanes 0-127
-                float acc[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + tile * 16, acc);
-                const int row = tile * TM + warp * 32 + lane;   // (tap, ci) = (row / 16, row % 16)
+    for (int tile = 0; tile < WG_MT; tile++) {
+        const int row = tile * TM + warp * 32 + lane;   // (tap, ci) = (row / 16, row % 16)
+        if (warp < 4) {   // warps 0-3 own TMEM lanes 0-127
+            float acc[16];
+            tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + tile * 16, acc);
+            float4 *o = reinterpret_cast<float4 *>(p + (size_t)row * CH);
+            if (row < NTAP * CH) {
 #pragma unroll
-                for (int co = 0; co < 16; co++) p[(size_t)row * CH + co] = acc[co];
+                for (int co = 0; co < 4; co++)
+                    o[co] = make_float4(acc[4 * co], acc[4 * co + 1], acc[4 * co + 2], acc[4 * co + 3]);
             }
         }
-    } else {
-        for (int t = tid; t < WG_MT * TM * CH; t += WG_NT) p[t] = 0.f;
     }
     tc::fence_before();
     __syncthreads();
