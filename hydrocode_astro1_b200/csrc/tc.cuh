@@ -26,6 +26,18 @@ __host__ __device__ __forceinline__ uint32_t kmajor_off(int r, int k, int KC)
     return (uint32_t)((r >> 3) * (16 * KC) + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
+// True in one thread of a converged warp.  MMAs are issued under this, not
+// under a test of the thread index: the compiler then knows that one thread
+// runs and keeps descriptors where the instruction takes them, and a stream of
+// M = 128, N = 16 MMAs runs at the tensor core's 39 cycles each (M = 64: 23)
+// instead of the 45 to 53 that a thread-index branch takes to issue one.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // One full warp executes alloc and dealloc.  ncols: power of two >= 32.
 __device__ __forceinline__ void tmem_alloc(uint32_t *smem_dst, uint32_t ncols)
 {

@@ -105,18 +105,27 @@ cudaError_t conv3(const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *b
     return cudaGetLastError();
 }
 
-// partial: nparts * WG_MT*TM*CH floats, nparts <= max_parts
+// partial: nparts * WG_MT*TM*CH floats, nparts <= max_parts.  Both kernels
+// add the same groups of voxels in the same order over the same parts.
 cudaError_t wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dy, float *dw, float *partial, int max_parts,
                   const Dims &d, int *err, cudaStream_t s)
 {
-    static std::atomic<unsigned long long> attr_set{0};
-    cudaError_t e = hc::set_smem_once(attr_set, (const void *)wgrad_kernel, (int)sizeof(WgradSmem));
-    if (e != cudaSuccess) return e;
     const long long nchunk = (d.n + KC - 1) / KC;
     int parts = (int)std::min<long long>(max_parts, nchunk);
     const int per = (int)((nchunk + parts - 1) / parts);
     parts = (int)((nchunk + per - 1) / per);
-    wgrad_kernel<<<parts, WG_NT, sizeof(WgradSmem), s>>>(x, dy, partial, d, per, err);
+    WrowGeom g;
+    if (wrow_geom(d, per, &g)) {
+        static std::atomic<unsigned long long> attr_set{0};
+        cudaError_t e = hc::set_smem_once(attr_set, (const void *)wgrad_row_kernel, (int)WR_SMEM);
+        if (e != cudaSuccess) return e;
+        wgrad_row_kernel<<<parts, WR_NT, g.smem(), s>>>(x, dy, partial, d, g, per, err);
+    } else {
+        static std::atomic<unsigned long long> attr_set{0};
+        cudaError_t e = hc::set_smem_once(attr_set, (const void *)wgrad_kernel, (int)sizeof(WgradSmem));
+        if (e != cudaSuccess) return e;
+        wgrad_kernel<<<parts, WG_NT, sizeof(WgradSmem), s>>>(x, dy, partial, d, per, err);
+    }
     wgrad_reduce_kernel<<<(WELEM + 255) / 256, 256, 0, s>>>(partial, parts, dw);
     return cudaGetLastError();
 }

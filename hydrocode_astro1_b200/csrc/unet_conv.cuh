@@ -187,13 +187,13 @@ conv3_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
 }
 
 // ---------------------------------------------------------------- weight gradient
-constexpr int WG_NT = 256;
+constexpr int WG_LT = 256, WG_NT = WG_LT + 32;   // loading threads, and a warp that issues
 constexpr int WG_MT = 4;                   // 128-row tiles: taps 0-7, 8-15, 16-23, 24-26
 constexpr int WG_ST = 3;                   // chunks staged in shared memory
 struct WgradSmem {
     __align__(128) unsigned char a[WG_ST][WG_MT][TM * KC * 2];   // 3 x 4 x 16 KB
     __align__(128) unsigned char b[WG_ST][CH * KC * 2];          // 3 x 2 KB
-    __align__(8) uint64_t bar[WG_ST];
+    __align__(8) uint64_t full[WG_ST], done[WG_ST];
     uint32_t tmem;
 };
 
@@ -209,6 +209,14 @@ __device__ __forceinline__ void cp16(unsigned char *dst, const __nv_bfloat16 *sr
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(in ? 16 : 0)
                  : "memory");
+}
+
+// Arrive on `bar` when this thread's cp.async so far have landed.  The thread
+// that waits on it fences for the tensor core: a proxy fence here would wait
+// for all copies in flight, a memory latency per chunk.
+__device__ __forceinline__ void arrive_async(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
 }
 
 // Taps G, G+2, ... of one voxel and channel half into the A tiles of a stage;
@@ -255,16 +263,18 @@ __device__ __forceinline__ void wgrad_fetch(WgradSmem &sm, int st, const __nv_bf
 // written and 72 KB read by the MMAs per chunk, about 1000 cycles.  Chunks are
 // fetched by cp.async two ahead of the one the tensor core works on; a warp
 // takes 16 voxels x 2 halves, 512 contiguous bytes.  Rows of taps past 26 are
-// never written and never read back.  128^3 voxels 1650 -> 261 us, 64^3 205 ->
-// 37 us against fetching through registers one chunk at a time, with a 64-bit
-// division chain per 16 bytes.
+// never written and never read back.  128^3 voxels 1650 -> 209 us, 64^3 205 ->
+// 32 us against fetching through registers one chunk at a time, with a 64-bit
+// division chain per 16 bytes.  One thread of a warp of its own issues, after
+// the one proxy fence, and elected: with the fence in the loading threads and a
+// thread-index test 128^3 stayed at 261 us.
 __global__ void __launch_bounds__(WG_NT)
 wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy, float *__restrict__ partial,
              Dims d, int chunks_per_cta, int *err)
 {
     extern __shared__ __align__(128) unsigned char smraw[];
     WgradSmem &sm = *reinterpret_cast<WgradSmem *>(smraw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const long long nchunk = (d.n + KC - 1) / KC;
     const long long c0 = (long long)blockIdx.x * chunks_per_cta;
     const int nq = (int)(min(nchunk, c0 + chunks_per_cta) - c0);
@@ -275,46 +285,49 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
         tc::fence_before();
     }
     if (tid == 0)
-        for (int q = 0; q < WG_ST; q++) tc::bar_init(&sm.bar[q], 1);
+        for (int q = 0; q < WG_ST; q++) {
+            tc::bar_init(&sm.full[q], WG_LT);
+            tc::bar_init(&sm.done[q], 1);
+        }
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = sm.tmem;
     constexpr uint32_t IDESC = tc::idesc_bf16(TM, CH) | (1u << 15) | (1u << 16);
     bool ok = true;
 
-    for (int q = -2; q < nq; q++) {   // q < 0: the first two fetches
-        if (q >= 0) {
+    if (warp < WG_LT / 32) {
+        for (int q = 0; q < nq; q++) {
             const int st = q % WG_ST;
-            asm volatile("cp.async.wait_group 1;" ::: "memory");   // all but the chunk after this one
+            if (q >= WG_ST) ok = tc::bar_wait(&sm.done[st], (q / WG_ST - 1) & 1) && ok;
+            const long long v = (c0 + q) * KC + kk;
+            if (warp < 4) wgrad_fetch<0>(sm, st, x, dy, d, v, kk, half);
+            else wgrad_fetch<1>(sm, st, x, dy, d, v, kk, half);
+            arrive_async(&sm.full[st]);
+        }
+    } else if (tc::elect_one()) {
+        for (int q = 0; q < nq; q++) {
+            const int st = q % WG_ST;
+            ok = tc::bar_wait(&sm.full[st], (q / WG_ST) & 1) && ok;
             tc::fence_smem_to_async();
-            __syncthreads();
-            if (tid == 0) {
-                tc::fence_after();
-                const uint32_t sb = tc::smem_u32(sm.b[st]);
+            tc::fence_after();
+            const uint32_t sb = tc::smem_u32(sm.b[st]);
 #pragma unroll
-                for (int tile = 0; tile < WG_MT; tile++) {
-                    const uint32_t sa = tc::smem_u32(sm.a[st][tile]);
+            for (int tile = 0; tile < WG_MT; tile++) {
+                const uint32_t sa = tc::smem_u32(sm.a[st][tile]);
 #pragma unroll
-                    for (int s = 0; s < 4; s++) {
-                        const uint64_t da = tc::sdesc(sa + s * 256, 128, 16 * KC);
-                        const uint64_t db = tc::sdesc(sb + s * 256, 128, 16 * KC);
-                        tc::mma_bf16(tmem + tile * 16, da, db, IDESC, (q > 0 || s > 0) ? 1u : 0u);
-                    }
+                for (int s = 0; s < 4; s++) {
+                    const uint64_t da = tc::sdesc(sa + s * 256, 128, 16 * KC);
+                    const uint64_t db = tc::sdesc(sb + s * 256, 128, 16 * KC);
+                    tc::mma_bf16(tmem + tile * 16, da, db, IDESC, (q > 0 || s > 0) ? 1u : 0u);
                 }
-                tc::mma_commit(&sm.bar[st]);
             }
-            // the stage of chunk q + 2 is that of q - 1
-            if (q >= 1) ok = tc::bar_wait(&sm.bar[(q - 1) % WG_ST], ((q - 1) / WG_ST) & 1) && ok;
+            tc::mma_commit(&sm.done[st]);
         }
-        if (q + 2 < nq) {
-            const long long v = (c0 + q + 2) * KC + kk;
-            if (warp < 4) wgrad_fetch<0>(sm, (q + 2) % WG_ST, x, dy, d, v, kk, half);
-            else wgrad_fetch<1>(sm, (q + 2) % WG_ST, x, dy, d, v, kk, half);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    __syncthreads();
     float *p = partial + (size_t)blockIdx.x * (WG_MT * TM * CH);
-    ok = tc::bar_wait(&sm.bar[(nq - 1) % WG_ST], ((nq - 1) / WG_ST) & 1) && ok;   // the last commit covers all
+    ok = tc::bar_wait(&sm.done[(nq - 1) % WG_ST], ((nq - 1) / WG_ST) & 1) && ok;   // the last commit covers all
+    __syncwarp();
     tc::fence_after();
 #pragma unroll
     for (int tile = 0; tile < WG_MT; tile++) {
@@ -333,7 +346,7 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 64);
-    if (!ok && tid == 0) atomicExch(err, -6);
+    if (!ok) atomicExch(err, -6);
 }
 
 // dW[co][tap][ci] = sum over CTAs of partial[cta][tap*16+ci][co], fixed order
@@ -509,6 +522,199 @@ conv3_halo_kernel(const __grid_constant__ CUtensorMap tmx, const __nv_bfloat16 *
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 32);
     if (!ok && tid == 0) atomicExch(err, -6);
+}
+
+// ---------------------------------------------------------------------------
+// Weight gradient without shifted copies, for rows of a multiple of 16 voxels.
+//
+// A CTA walks its voxels row by row.  Rows j-1, j, j+1 of planes i-1, i, i+1
+// live in a ring of slots, each {row j of three planes}, with one voxel of halo
+// at both ends (zeros outside the volume), laid out [half][plane][k][8 ch]: for
+// MMAs that contract over 16 voxels the 6 groups (half, plane) are rows 0-47 of
+// an MN-major A operand with one stride, and the tap's shift along k is 16 bytes
+// of the descriptor's start.  So 16 voxels are 9 MMAs (M = 64: three planes x 16
+// channels and two groups of whatever follows, never read back; N = 16), one per
+// (tap j, tap k), and stepping j loads only one new slot.  The voxels are grouped
+// and added up in the order of wgrad_kernel over the same ranges: the bits are
+// the same.
+//
+// Five warps fetch by cp.async, row by row in turn.  Three threads issue, one
+// per tap j, each into accumulators of its own: one thread spends 670 cycles
+// between the last MMA of a row and the first of the next, and the tensor core
+// waits for it.
+//
+// What bounds it is the rate of these MMAs, 23 cycles each (17 of them to read
+// the 64 rows of A from shared memory), 13 per voxel.  128^3 voxels 209 us
+// (wgrad_kernel) -> 112, 96^3 94 -> 52, 64^3 32 -> 22.
+// ---------------------------------------------------------------------------
+constexpr int WR_NT = 256, WR_LW = 5;      // threads; loading warps (the last three issue, one per tap j)
+constexpr int WR_MAXS = 10, WR_MINS = 4;   // slots: three in use, the rest ahead
+constexpr int WR_RING = 16;                // > slots: rows between the loaders and the issuer
+constexpr unsigned WR_SMEM = 227 * 1024;
+
+struct WrowBars {
+    uint64_t ready[WR_RING], done[WR_RING], fin;
+    uint32_t tmem;
+};
+
+struct WrowGeom {
+    int kb, slots, dys;                    // voxels of a row with its halo, ring slots, rows of dY staged
+    unsigned slot_bytes, dy_bytes;
+    // the two groups past the last slot's planes fall into the rows of dY
+    __host__ __device__ unsigned bars_at() const { return slots * slot_bytes + dys * dy_bytes; }
+    __host__ __device__ unsigned smem() const { return bars_at() + (unsigned)sizeof(WrowBars); }
+};
+
+// Whether wgrad_row_kernel takes a volume, `per_cta` chunks to a CTA.  Not rows
+// of odd lengths (a group of 16 voxels would span rows), short ones (256 x 256 x
+// 16: 151 us against 106; 32^3: 9.8 against 8.8; 48^3: 13.7 against 15.9), and
+// CTAs of a few rows, which fetch mostly neighbours (16 x 16 x 384, two rows:
+// 20 against 16; 32 x 32 x 256, seven: 24 against 31).
+__host__ inline bool wrow_geom(const Dims &d, int per_cta, WrowGeom *g)
+{
+    if (d.nz % 16 || d.nz < 48 || d.nz > 1024 || (long long)per_cta * KC < 4LL * d.nz) return false;
+    g->kb = d.nz + 2;
+    g->slot_bytes = 96u * g->kb;
+    g->dy_bytes = 32u * d.nz;
+    for (g->slots = WR_MAXS; g->slots >= WR_MINS; g->slots--) {
+        g->dys = g->slots - 2;
+        if (g->smem() <= WR_SMEM) return true;
+    }
+    return false;                          // rows past 512 leave no room for four slots
+}
+
+// partial[cta][tap][ci][co] over the voxels of chunks [c0, c1), as wgrad_kernel
+__global__ void __launch_bounds__(WR_NT)
+wgrad_row_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy, float *__restrict__ partial,
+                 Dims d, WrowGeom g, int chunks_per_cta, int *err)
+{
+    extern __shared__ __align__(128) unsigned char smraw[];
+    WrowBars &sm = *reinterpret_cast<WrowBars *>(smraw + g.bars_at());
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const long long v0 = (long long)blockIdx.x * chunks_per_cta * KC;
+    const long long v1 = min(d.n, v0 + (long long)chunks_per_cta * KC);
+    const long long row0 = v0 / d.nz;
+    const int nu = (int)((v1 - 1) / d.nz - row0) + 1;              // rows touched
+    const int kfirst = (int)(v0 - row0 * d.nz), klast = (int)(v1 - (row0 + nu - 1) * d.nz);
+    const int i0 = (int)(row0 / d.ny), j0 = (int)(row0 % d.ny);
+
+    if (warp == 0) {
+        tc::tmem_alloc(&sm.tmem, 256);
+        tc::fence_before();
+    }
+    if (tid == 0) {
+        for (int q = 0; q < WR_RING; q++) {
+            tc::bar_init(&sm.ready[q], 32);
+            tc::bar_init(&sm.done[q], 3);
+        }
+        tc::bar_init(&sm.fin, 3);
+    }
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = sm.tmem, sx = tc::smem_u32(smraw), sy = sx + g.slots * g.slot_bytes;
+    bool ok = true;
+
+    if (warp < WR_LW) {
+        // Row u needs loads ell(u) .. ell(u) + 2, ell stepping by 1 within a plane and by 3 into the next.  Loading
+        // warps take rows in turn: one row's loads are a chain of a thousand cycles and more.
+        int ld = 0, slot = 0, w = -1, wj = j0 - 1, well = -1;      // w: last row known to be done, its j and ell
+        int i = i0, j = j0;
+        const int half = (lane >> 3) & 1, kl = (lane >> 4) * 8 + (lane & 7);   // 8 voxels of one half, then the other
+        for (int u = 0; u < nu; u++) {
+            const int jfrom = (u == 0 || j == 0) ? j - 1 : j + 1, nl = j + 2 - jfrom;
+            const bool mine = u % WR_LW == warp;
+            if (mine) {
+                // rows still reading what the new loads and the row of dY replace
+                const int w0 = w;
+                for (;;) {
+                    const int next = w < 0 ? 0 : wj + 1 == d.ny ? well + 3 : well + 1;
+                    if (w + 1 >= u || (next > ld + nl - 1 - g.slots && w + 1 > u - g.dys)) break;
+                    w++;
+                    well = next;
+                    if (++wj == d.ny) wj = 0;
+                }
+                if (w > w0) ok = tc::bar_wait(&sm.done[w % WR_RING], (w / WR_RING) & 1) && ok;
+                __syncwarp();
+            }
+            for (int jj = jfrom; jj <= j + 1; jj++) {
+                if (mine) {
+                    const bool in_j = jj >= 0 && jj < d.ny;
+#pragma unroll
+                    for (int a = 0; a < 3; a++) {
+                        const int ii = i + a - 1;
+                        const bool in = in_j && ii >= 0 && ii < d.nx;
+                        const __nv_bfloat16 *src = in ? x + ((long long)ii * d.ny + jj) * d.nz * CH + half * 8 - CH : x;
+                        unsigned char *dst = smraw + slot * g.slot_bytes + (a + 3 * half) * 16 * g.kb;
+#pragma unroll 4
+                        for (int k = kl; k < g.kb; k += 16) {      // k: voxel k - 1
+                            const bool there = in && k > 0 && k <= d.nz;
+                            cp16(dst + k * 16, there ? src + k * CH : x, there);
+                        }
+                    }
+                }
+                ld++;
+                if (++slot == g.slots) slot = 0;
+            }
+            if (mine) {
+                const __nv_bfloat16 *src = dy + ((long long)i * d.ny + j) * d.nz * CH + half * 8;
+                unsigned char *dst = smraw + g.slots * g.slot_bytes + (u % g.dys) * g.dy_bytes + half * 16 * d.nz;
+#pragma unroll 4
+                for (int k = kl; k < d.nz; k += 16) cp16(dst + k * 16, src + k * CH, true);
+                arrive_async(&sm.ready[u % WR_RING]);
+            }
+            if (++j == d.ny) j = 0, i++;
+        }
+    } else if (tc::elect_one()) {
+        constexpr uint32_t IDESC = tc::idesc_bf16(64, CH) | (1u << 15) | (1u << 16);
+        const int b = warp - WR_LW;        // tap j
+        const uint64_t xd = tc::sdesc(sx, 128, 16 * g.kb), yd = tc::sdesc(sy, 128, 16 * d.nz);
+        const uint32_t acc0 = tmem + b * 3 * 16;
+        int slot = b, j = j0, dyr = 0;     // slot of load ell + b
+        uint32_t acc = 0;
+        for (int u = 0; u < nu; u++) {
+            const uint64_t xb = xd + (slot * g.slot_bytes >> 4), yb = yd + (dyr * g.dy_bytes >> 4);
+            const int ke = u == nu - 1 ? klast : d.nz;
+            ok = tc::bar_wait(&sm.ready[u % WR_RING], (u / WR_RING) & 1) && ok;
+            tc::fence_smem_to_async();
+            tc::fence_after();
+            for (int k = u == 0 ? kfirst : 0; k < ke; k += 16) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) tc::mma_bf16(acc0 + c * 16, xb + k + c, yb + k, IDESC, acc);
+                acc = 1;
+            }
+            tc::mma_commit(&sm.done[u % WR_RING]);
+            const int step = ++j == d.ny ? 3 : 1;
+            if (j == d.ny) j = 0;
+            slot += step;
+            if (slot >= g.slots) slot -= g.slots;
+            if (++dyr == g.dys) dyr = 0;
+        }
+        tc::mma_commit(&sm.fin);
+    }
+    __syncthreads();
+    ok = tc::bar_wait(&sm.fin, 0) && ok;
+    __syncwarp();
+    tc::fence_after();
+    if (warp < 4) {
+        // M = 64: row r lies in TMEM lane 32 (r / 16) + r % 16
+        const int r = warp * 16 + (lane & 15), half = r / 24, a = (r % 24) >> 3, ci = half * 8 + (r & 7);
+        float *p = partial + (size_t)blockIdx.x * (WG_MT * TM * CH);
+#pragma unroll
+        for (int bc = 0; bc < 9; bc++) {
+            float v[16];
+            tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + bc * 16, v);
+            if (lane < 16 && r < 48) {
+                float4 *o = reinterpret_cast<float4 *>(p + (size_t)((a * 9 + bc) * CH + ci) * CH);
+#pragma unroll
+                for (int co = 0; co < 4; co++)
+                    o[co] = make_float4(v[4 * co], v[4 * co + 1], v[4 * co + 2], v[4 * co + 3]);
+            }
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, 256);
+    if (!ok) atomicExch(err, -6);
 }
 
 }  // namespace unet
