@@ -126,7 +126,7 @@ cudaError_t wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dy, float *dw, fl
         if (e != cudaSuccess) return e;
         wgrad_kernel<<<parts, WG_NT, sizeof(WgradSmem), s>>>(x, dy, partial, d, per, err);
     }
-    wgrad_reduce_kernel<<<(WELEM + 255) / 256, 256, 0, s>>>(partial, parts, dw);
+    wgrad_reduce_kernel<<<(WELEM + WRED_NT - 1) / WRED_NT, WRED_NT, 0, s>>>(partial, parts, dw);
     return cudaGetLastError();
 }
 
@@ -251,8 +251,7 @@ void full_to_compact(const std::vector<float> &f, float *c)
 
 cudaError_t pack_all(UNetState *u, cudaStream_t s)
 {
-    for (int l = 0; l < NCONV; l++)
-        pack_weights_kernel<<<(WELEM + 255) / 256, 256, 0, s>>>(u->pm + (size_t)l * PFULL, wf_of(u, l), wt_of(u, l));
+    pack_weights_kernel<<<dim3((WELEM + 255) / 256, NCONV), 256, 0, s>>>(u->pm, PFULL, wf_of(u, 0), wt_of(u, 0));
     return cudaGetLastError();
 }
 

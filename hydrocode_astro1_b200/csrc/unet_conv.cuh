@@ -349,16 +349,33 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
     if (!ok) atomicExch(err, -6);
 }
 
-// dW[co][tap][ci] = sum over CTAs of partial[cta][tap*16+ci][co], fixed order
-__global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int nparts, float *__restrict__ dw)
+// The sum of n values `stride` apart in their order, 16 loads in flight: with
+// one add per load the chain is n memory latencies.  (37 with the last batch
+// masked is slower: the masks cost more than the fewer latencies save.)
+__device__ __forceinline__ float sum_in_order(const float *__restrict__ p, int n, int stride)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;   // (co, tap, ci)
-    if (e >= WELEM) return;
-    const int co = e / (NTAP * CH), tap = (e / CH) % NTAP, ci = e % CH;
-    const int row = tap * CH + ci;
     float s = 0.f;
-    for (int p = 0; p < nparts; p++) s += partial[(size_t)p * (WG_MT * TM * CH) + (size_t)row * CH + co];
-    dw[e] = s;
+    int q = 0;
+    for (; q + 16 <= n; q += 16) {
+        float f[16];
+#pragma unroll
+        for (int t = 0; t < 16; t++) f[t] = p[(size_t)(q + t) * stride];
+#pragma unroll
+        for (int t = 0; t < 16; t++) s += f[t];
+    }
+    for (; q < n; q++) s += p[(size_t)q * stride];
+    return s;
+}
+
+// dW[co][tap][ci] = sum over CTAs of partial[cta][tap*16+ci][co], fixed order.
+// Neighbouring threads read neighbouring co (15 -> 9.5 us for 148 parts).
+constexpr int WRED_NT = 64;
+__global__ void __launch_bounds__(WRED_NT) wgrad_reduce_kernel(const float *__restrict__ partial, int nparts,
+                                                               float *__restrict__ dw)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;   // (tap, ci, co)
+    if (e >= WELEM) return;
+    dw[(size_t)(e % CH) * (NTAP * CH) + e / CH] = sum_in_order(partial + e, nparts, WG_MT * TM * CH);
 }
 
 
