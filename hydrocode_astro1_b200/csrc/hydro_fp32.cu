@@ -52,9 +52,8 @@ cudaError_t fp32_dt(const HydroArgs &a, cudaStream_t s)
 }
 
 // TMA tensor map over the five FP32 fields of a state buffer:
-// dims (k, j, i, field), box (40, 10, planes, 5) -- one (planes = 1) or two
-// (planes = 2) plane tiles with halo.
-static cudaError_t encode_state_map(const HydroArgs &a, CUtensorMap *tm, unsigned planes = 1)
+// dims (k, j, i, field), box (rk, rj, planes, 5): the kernel's tile with halo.
+static cudaError_t encode_state_map(const HydroArgs &a, CUtensorMap *tm, int rk, int rj, unsigned planes)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
     if (!enc) {
@@ -67,7 +66,7 @@ static cudaError_t encode_state_map(const HydroArgs &a, CUtensorMap *tm, unsigne
     const cuuint64_t n = (cuuint64_t)a.g.n;
     cuuint64_t dims[4] = { (cuuint64_t)a.g.nz, (cuuint64_t)a.g.ny, (cuuint64_t)a.g.nx, 5 };
     cuuint64_t strides[3] = { (cuuint64_t)a.g.nz * 4, (cuuint64_t)a.g.ny * a.g.nz * 4, n * 4 };
-    cuuint32_t box[4] = { (cuuint32_t)tma32::RK, (cuuint32_t)tma32::RJ, planes, 5 };
+    cuuint32_t box[4] = { (cuuint32_t)rk, (cuuint32_t)rj, planes, 5 };
     cuuint32_t es[4] = { 1, 1, 1, 1 };
     CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void *>(a.qin[0]), dims, strides, box,
                      es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -126,7 +125,7 @@ static int pk_chunks(long long tiles, int nint, long long slots)
 static cudaError_t pk_interior(const HydroArgs &a, cudaStream_t s)
 {
     CUtensorMap tm;
-    cudaError_t e = encode_state_map(a, &tm, 2);
+    cudaError_t e = encode_state_map(a, &tm, pk::RK, pk::RJ, 2);
     if (e != cudaSuccess) return e;
     static std::atomic<unsigned long long> attr_set{0};
     e = set_smem_once(attr_set, (const void *)pk::interior_pk_kernel, (int)pk::SMEM);
@@ -164,7 +163,7 @@ cudaError_t fp32_interior(const HydroArgs &a, cudaStream_t s)
     }
     if (hydro32_choice() <= 1 && tma_usable(a)) {
         CUtensorMap tm;
-        cudaError_t e = encode_state_map(a, &tm);
+        cudaError_t e = encode_state_map(a, &tm, tma32::RK, tma32::RJ, 1);
         if (e == cudaSuccess) {
             // 4 CTAs per SM, about 4 waves
             long long tiles = (long long)((a.g.nz + tma32::TK - 1) / tma32::TK) * ((a.g.ny + tma32::TJ - 1) / tma32::TJ);

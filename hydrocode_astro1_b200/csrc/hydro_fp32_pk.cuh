@@ -16,7 +16,7 @@
 //     copy starts on a 16-byte boundary) into a double buffer, one pair
 //     ahead, completing on an mbarrier with bounded waits.
 //   * The y and z faces of a pair are natural pairs: (plane i, plane i+1) at
-//     the same (j, k).  Cell records live in shared memory as six float4
+//     the same (j, k).  Cell records live in shared memory as four float4
 //     planes of structure-of-arrays (conflict-free 16-byte accesses, each
 //     carrying both planes of two quantities); face fluxes likewise.
 //   * The x faces i+1/2 and i+3/2 of the pair are the packed HLLC of the
@@ -50,7 +50,7 @@ constexpr int NH = 2 * SK + 2 * TJ;   // halo records around the tile
 // shared-memory layout (bytes)
 constexpr size_t OFF_RAW = 0;
 constexpr size_t OFF_P = OFF_RAW + 2 * (size_t)RAW_BYTES;
-constexpr size_t OFF_FYA = OFF_P + 6 * (size_t)NS * 16;
+constexpr size_t OFF_FYA = OFF_P + 4 * (size_t)NS * 16;
 constexpr size_t OFF_FYB = OFF_FYA + (size_t)NFY * 16;
 constexpr size_t OFF_FYE = OFF_FYB + (size_t)NFY * 16;
 constexpr size_t OFF_FZA = OFF_FYE + (size_t)NFY * 8;
@@ -126,15 +126,16 @@ __device__ __forceinline__ R2 rec_raw(const float *r, int o, const Consts &K)
                      make_float2(r[8 * RAWF + o], r[9 * RAWF + o]), K);
 }
 
-// shared records: six float4 planes of NS each
+// shared records: four float4 planes of NS each; the floored density and the
+// velocity that a face needs are formed again by the operations that made them
+// (with them in two more planes: 308 us per 256^3 step
+// against 294)
 __device__ __forceinline__ void put_rec(float4 *P, int s, const R2 &r)
 {
     P[s] = make_float4(r.d.x, r.d.y, r.mx.x, r.mx.y);
     P[NS + s] = make_float4(r.my.x, r.my.y, r.mz.x, r.mz.y);
-    P[2 * NS + s] = make_float4(r.E.x, r.E.y, r.u.x, r.u.y);
-    P[3 * NS + s] = make_float4(r.v.x, r.v.y, r.w.x, r.w.y);
-    P[4 * NS + s] = make_float4(r.p.x, r.p.y, r.c.x, r.c.y);
-    P[5 * NS + s] = make_float4(r.dh.x, r.dh.y, r.inv.x, r.inv.y);
+    P[2 * NS + s] = make_float4(r.E.x, r.E.y, r.p.x, r.p.y);
+    P[3 * NS + s] = make_float4(r.c.x, r.c.y, r.inv.x, r.inv.y);
 }
 __device__ __forceinline__ R2 get_rec(const float4 *P, int s)
 {
@@ -144,13 +145,13 @@ __device__ __forceinline__ R2 get_rec(const float4 *P, int s)
     t = P[NS + s];
     r.my = make_float2(t.x, t.y); r.mz = make_float2(t.z, t.w);
     t = P[2 * NS + s];
-    r.E = make_float2(t.x, t.y); r.u = make_float2(t.z, t.w);
+    r.E = make_float2(t.x, t.y); r.p = make_float2(t.z, t.w);
     t = P[3 * NS + s];
-    r.v = make_float2(t.x, t.y); r.w = make_float2(t.z, t.w);
-    t = P[4 * NS + s];
-    r.p = make_float2(t.x, t.y); r.c = make_float2(t.z, t.w);
-    t = P[5 * NS + s];
-    r.dh = make_float2(t.x, t.y); r.inv = make_float2(t.z, t.w);
+    r.c = make_float2(t.x, t.y); r.inv = make_float2(t.z, t.w);
+    r.dh = maxs2(r.d, (float)HC_RHO_FLOOR);
+    r.u = mul2(r.mx, r.inv);
+    r.v = mul2(r.my, r.inv);
+    r.w = mul2(r.mz, r.inv);
     return r;
 }
 __device__ __forceinline__ void put_flux(float4 *A, float4 *B, float2 *E, int s, const F2 &f)
@@ -201,12 +202,14 @@ __device__ __forceinline__ F2 hllc2(const R2 &L, const R2 &R)
     const bool supr_x = !supl_x && sR.x <= 0.f, supr_y = !supl_y && sR.y <= 0.f;
     const bool lx = supl_x || (!supr_x && ss.x >= 0.f), ly = supl_y || (!supr_y && ss.y >= 0.f);
     const bool starx = !(supl_x || supr_x), stary = !(supl_y || supr_y);
-    const float2 sK = sel2(lx, ly, sL, sR), uK = sel2(lx, ly, uL, uR);
-    const float2 gK = sel2(lx, ly, gL, gR), qK = sel2(lx, ly, qL, qR);
+    const float2 sK = sel2(lx, ly, sL, sR), qK = sel2(lx, ly, qL, qR);
     const float2 pK = sel2(lx, ly, L.p, R.p), iK = sel2(lx, ly, L.inv, R.inv);
     const float2 EK = sel2(lx, ly, L.E, R.E), dK = sel2(lx, ly, L.d, R.d);
     const float2 mxK = sel2(lx, ly, L.mx, R.mx), myK = sel2(lx, ly, L.my, R.my), mzK = sel2(lx, ly, L.mz, R.mz);
-    const float2 vxK = sel2(lx, ly, L.u, R.u), vyK = sel2(lx, ly, L.v, R.v), vzK = sel2(lx, ly, L.w, R.w);
+    // (the side's velocities and S - u again by the packed operations that made
+    // them, the same bits: a select is per face; 320 -> 308 us per 256^3 step)
+    const float2 vxK = mul2(mxK, iK), vyK = mul2(myK, iK), vzK = mul2(mzK, iK);
+    const float2 uK = A == 0 ? vxK : (A == 1 ? vyK : vzK), gK = sub2(sK, uK);
     // star-region weight: S_K inside, 0 outside (then F = F_K exactly)
     const float2 zero = sp2(0.f);
     const float2 sKw = sel2(starx, stary, sK, zero);
