@@ -83,15 +83,22 @@ __device__ __forceinline__ CellS<T> make_cell(const Cons<T> &q, T gm1, T gam)
 // --------------------------------------------------------------------------
 // interior kernel
 // --------------------------------------------------------------------------
+// In FP64 the chains of divisions and square roots of the primitives and the
+// faces bound it (about 29 divisions per cell), so no cell of a tile is turned
+// into primitives twice: the thread that owns it keeps it for the x face and
+// posts it, and a halo cell has a thread of its own.  Its loads run during the
+// y and z faces.  Two blocks to an SM (128 registers): at 138 one fits, three
+// spill.  256^3 1550 -> 1063 us against forming tile and halo from a staged raw
+// plane, 128^3 220 -> 155, 90 x 101 x 97 115 -> 77, 64^3 39 -> 31; tiles of 4
+// rows 5 % and of 16 rows 1 % slower at 256^3.
 template <typename T, int TK, int TJ>
-__global__ void __launch_bounds__(TK * TJ)
+__global__ void __launch_bounds__(TK * TJ, 2)
 interior_kernel(HydroArgs a, int ilen, int k00, int j00)   // k00, j00: first cell of the tiles
 {
     constexpr int SK = TK + 2, SJ = TJ + 2, NS = SK * SJ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CellS<T> *P = reinterpret_cast<CellS<T> *>(smem_raw);            // plane i, tile+halo
-    Cons<T> *Qn = reinterpret_cast<Cons<T> *>(P + NS);                 // plane i+1 raw
-    Cons<T> *FY = Qn + NS;                                              // (TJ+1) x TK
+    Cons<T> *FY = reinterpret_cast<Cons<T> *>(P + NS);                 // (TJ+1) x TK
     Cons<T> *FZ = FY + (TJ + 1) * TK;                                   // TJ x (TK+1)
 
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
@@ -112,63 +119,66 @@ interior_kernel(HydroArgs a, int ilen, int k00, int j00)   // k00, j00: first ce
     const bool own_in = (j < ny) && (k < nz);
     const bool own_int = (j >= 1) && (j <= ny - 2) && (k >= 1) && (k <= nz - 2);
 
-    auto load_plane = [&](int i, Cons<T> *dst) {
-        for (int s = tid; s < NS; s += TK * TJ) {
-            int sj = s / SK, sk = s - sj * SK;
-            int gj = j0 - 1 + sj, gk = k0 - 1 + sk;
-            Cons<T> q;
-            if (gj >= 0 && gj < ny && gk >= 0 && gk < nz) {
-                q = ld_cons(qin, (long long)i * sI + gj * sJ + gk);
-            } else {
-                q.d = (T)1; q.m[0] = q.m[1] = q.m[2] = (T)0; q.e = (T)1;
-            }
-            dst[s] = q;
+    // state of cell (gj, gk) of plane i; a harmless one outside the grid
+    auto load = [&](int i, int gj, int gk) {
+        Cons<T> q;
+        if (gj >= 0 && gj < ny && gk >= 0 && gk < nz) {
+            q = ld_cons(qin, (long long)i * sI + gj * sJ + gk);
+        } else {
+            q.d = (T)1; q.m[0] = q.m[1] = q.m[2] = (T)0; q.e = (T)1;
         }
+        return q;
     };
-    auto prims_plane = [&]() {
-        for (int s = tid; s < NS; s += TK * TJ) P[s] = make_cell(Qn[s], gm1, gam);
-    };
+    // One of the NH halo cells around the tile, for the last NH threads (the
+    // first two rows of threads form the faces behind the tile).
+    constexpr int NH = 2 * SK + 2 * TJ;
+    static_assert(NH <= TK * TJ, "a thread per halo cell");
+    const int h = tid - (TK * TJ - NH);
+    int hj = 0, hk = 0;
+    if (h >= 2 * SK) {
+        hj = 1 + ((h - 2 * SK) >> 1);
+        hk = (h & 1) ? SK - 1 : 0;
+    } else if (h >= 0) {
+        hj = h < SK ? 0 : SJ - 1;
+        hk = h % SK;
+    }
+    const int own = (ty + 1) * SK + tx + 1;
 
     // prologue: plane ib-1 (own cell only) and plane ib (tile + halo)
-    CellS<T> me_prev;
-    {
-        Cons<T> q;
-        if (own_in) q = ld_cons(qin, (long long)(ib - 1) * sI + j * sJ + k);
-        else { q.d = (T)1; q.m[0] = q.m[1] = q.m[2] = (T)0; q.e = (T)1; }
-        me_prev = make_cell(q, gm1, gam);
-    }
-    load_plane(ib, Qn);
-    __syncthreads();
-    prims_plane();
-    __syncthreads();
-    CellS<T> me = P[(ty + 1) * SK + tx + 1];
+    const CellS<T> me_prev = make_cell(load(ib - 1, j, k), gm1, gam);
+    CellS<T> me = make_cell(load(ib, j, k), gm1, gam);
+    P[own] = me;
+    if (h >= 0) P[hj * SK + hk] = make_cell(load(ib, j0 - 1 + hj, k0 - 1 + hk), gm1, gam);
     Cons<T> fxm = hllc<0>(me_prev.q, me_prev.w, me_prev.c, me.q, me.w, me.c);
+    __syncthreads();
 
     T smax = (T)0;
     for (int i = ib; i < ie; i++) {
-        // next plane raw state (tile + halo)
-        load_plane(i + 1, Qn);
-        __syncthreads();
-        CellS<T> nx1 = make_cell(Qn[(ty + 1) * SK + tx + 1], gm1, gam);
-        Cons<T> fxp = hllc<0>(me.q, me.w, me.c, nx1.q, nx1.w, nx1.c);
+        // plane i+1: this thread's cell and its halo cell, on their way during
+        // the faces of plane i
+        const Cons<T> qn = load(i + 1, j, k);
+        Cons<T> qh;
+        if (h >= 0) qh = load(i + 1, j0 - 1 + hj, k0 - 1 + hk);
         {
-            const CellS<T> &a0 = P[(ty + 1) * SK + tx + 1];
             const CellS<T> &ay = P[(ty + 2) * SK + tx + 1];
             const CellS<T> &az = P[(ty + 1) * SK + tx + 2];
-            FY[(ty + 1) * TK + tx] = hllc<1>(a0.q, a0.w, a0.c, ay.q, ay.w, ay.c);
-            FZ[ty * (TK + 1) + tx + 1] = hllc<2>(a0.q, a0.w, a0.c, az.q, az.w, az.c);
+            FY[(ty + 1) * TK + tx] = hllc<1>(me.q, me.w, me.c, ay.q, ay.w, ay.c);
+            FZ[ty * (TK + 1) + tx + 1] = hllc<2>(me.q, me.w, me.c, az.q, az.w, az.c);
             if (ty == 0) {
                 const CellS<T> &b0 = P[tx + 1];
-                FY[tx] = hllc<1>(b0.q, b0.w, b0.c, a0.q, a0.w, a0.c);
+                FY[tx] = hllc<1>(b0.q, b0.w, b0.c, me.q, me.w, me.c);
             } else if (ty == 1 && tx < TJ) {
                 const CellS<T> &c0 = P[(tx + 1) * SK];
                 const CellS<T> &c1 = P[(tx + 1) * SK + 1];
                 FZ[tx * (TK + 1)] = hllc<2>(c0.q, c0.w, c0.c, c1.q, c1.w, c1.c);
             }
         }
+        const CellS<T> nx1 = make_cell(qn, gm1, gam);
+        const Cons<T> fxp = hllc<0>(me.q, me.w, me.c, nx1.q, nx1.w, nx1.c);
         __syncthreads();
-        // P is free again: prepare plane i+1 for the next iteration
-        prims_plane();
+        // P is free again: plane i+1 for the next iteration
+        P[own] = nx1;
+        if (h >= 0) P[hj * SK + hk] = make_cell(qh, gm1, gam);
 
         if (own_in && own_int) {
             const Cons<T> &yp = FY[(ty + 1) * TK + tx], &ym = FY[ty * TK + tx];
@@ -207,13 +217,12 @@ interior_kernel(HydroArgs a, int ilen, int k00, int j00)   // k00, j00: first ce
 template <typename T, int TK, int TJ>
 constexpr size_t interior_smem()
 {
-    return sizeof(CellS<T>) * (TK + 2) * (TJ + 2) + sizeof(Cons<T>) * (TK + 2) * (TJ + 2) +
-           sizeof(Cons<T>) * ((TJ + 1) * TK + TJ * (TK + 1));
+    return sizeof(CellS<T>) * (TK + 2) * (TJ + 2) + sizeof(Cons<T>) * ((TJ + 1) * TK + TJ * (TK + 1));
 }
 
 // Planes of a chunk along i: the fewest waves x (planes + the prologue's one)
 // over the CTAs that run at once.  (A fixed four waves of at least 8 planes
-// left most SMs idle on small grids.  FP64, before -> now: 16^3 107 -> 19 us,
+// left most SMs idle on small grids.  FP64, by this rule alone: 16^3 107 -> 19 us,
 // 64^3 66 -> 40, 128^3 246 -> 220, 256^3 1664 -> 1550.)
 inline int chunk_planes(long long tiles, int nint, long long slots)
 {
