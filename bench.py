@@ -321,11 +321,18 @@ def reference_sample(q0, p, sor_iters=10):
 
 
 # DRAM bytes (read + write) per grid cell of one launch, from ncu captures of
-# the 256^3 workload (profiles/sor_split_vec_kernel_fp32_stellar_explosion_256.txt,
+# the 256^3 workload (profiles/sor_stream_kernel_fp32_stellar_explosion_256.txt,
 # profiles/sor_split_kernel_fp64_stellar_explosion_256.txt), keyed by kernel.
-NCU_DRAM_BYTES_PER_CELL = {"sor_split_vec_kernel": 6.47, "sor_split_kernel": 14.38}
-# the colour sweep each precision runs (FP32: 16-byte vector sweeps)
-SOR_KERNEL = {4: "sor_split_vec_kernel", 8: "sor_split_kernel"}
+NCU_DRAM_BYTES_PER_CELL = {"sor_stream_kernel": 12.45, "sor_split_kernel": 14.38}
+
+
+def sor_unit(word, iterations, launches):
+    """(kernel, iterations of one unit) of the default relaxation: a launch of
+    thousands of iterations of a grid resident in shared memory (counted per
+    iteration), an FP32 pass of two, an FP64 colour sweep."""
+    if 4 * launches < iterations:
+        return "sor_resident_kernel", 1.0
+    return ("sor_stream_kernel", 2.0) if word == 4 else ("sor_split_kernel", 0.5)
 
 REF_ITERS_FILE = os.path.join(ROOT, "hydrocode_astro1_b200", "data", "fp64_iterations.json")
 
@@ -420,29 +427,29 @@ def main_ours(args):
     s = r["solver"]
     fp64 = variant.startswith("fp64")
 
-    # roofline of the dominant kernel: one colour sweep of the colour-split SOR.
-    # Algorithmic bytes: half an iteration's 24 B/cell (FP64 phi read + write,
-    # rho read) or 12 B/cell (FP32 e read + write, r read) over the interior
-    # cells.  Launch time: the SOR family's CUDA-event time over the sweeps
-    # that ran (two per iteration); it also holds the convergence checks and
-    # the sweeps queued past convergence that return at once, so it is an
-    # upper bound of the sweep time.
+    # roofline of the dominant kernel, the relaxation's.  Algorithmic bytes of
+    # a unit: a pass of two FP32 iterations or one resident iteration 12 B/cell
+    # (e read + write, r read), an FP64 colour sweep half of 24 (phi read +
+    # write, rho read), over the interior cells.  Its time: the SOR family's
+    # CUDA-event time over the units that counted; it also holds the
+    # convergence checks and what was queued past convergence and returns at
+    # once, so it is an upper bound.
     interior = (p["shape"][0] - 2) * (p["shape"][1] - 2) * (p["shape"][2] - 2)
     word = 8 if fp64 else 4
-    bytes_per_launch = interior * 3 * word / 2.0
-    sweeps = max(2 * sum(r["iters"]), 1)
-    sor_avg_ms = tm["sor_ms"] / sweeps
+    kname, unit_its = sor_unit(word, sum(r["iters"]), tm["sor_launches"])
+    bytes_per_launch = interior * 3 * word * min(unit_its, 1.0)
+    units = max(sum(r["iters"]) / unit_its, 1)
+    sor_avg_ms = tm["sor_ms"] / units
     pk, pk_kind = peaks()
     achieved = bytes_per_launch / (sor_avg_ms / 1e3) / 1e9 if sor_avg_ms > 0 else 0.0
     shares = {k: tm[k] for k in ("hydro_ms", "bc_ms", "sor_ms", "residual_ms", "moments_ms", "unet_ms")}
-    kname = SOR_KERNEL[word]
     traffic = NCU_DRAM_BYTES_PER_CELL.get(kname)
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": pk, "unit": "GB/s",
                 "frac": achieved / pk, "peak_kind": pk_kind,
                 "traffic": traffic * ncell if traffic else None,
                 "algorithmic_bytes_per_launch": bytes_per_launch,
-                "layout_bytes_per_launch": 4 * word * ncell / 2.0,
-                "avg_launch_ms": sor_avg_ms, "sweeps": sweeps, "launches": tm["sor_launches"]}
+                "iterations_per_unit": unit_its,
+                "avg_launch_ms": sor_avg_ms, "units": units, "launches": tm["sor_launches"]}
     hydro_bytes = interior * (48 if not fp64 else 88)
     hydro_avg = tm["hydro_ms"] / max(tm["hydro_launches"], 1)
     hydro_roof = {"kernel": "hydro_interior", "achieved": hydro_bytes / (hydro_avg / 1e3) / 1e9 if hydro_avg else 0,

@@ -13,8 +13,9 @@ kernels, so an ncu capture of one of them starts at once.
 
 `sor`: two FP32 mixed-precision solves of the explosion's first state from
 a cold start, each capped at ITERATIONS correction iterations; prints the
-second solve's colour sweeps' time per iteration and algorithmic bandwidth
-(6 bytes per interior cell and sweep).
+second solve's time per iteration and algorithmic bandwidth (12 bytes per
+interior cell and iteration; a pass of two iterations moves them once, a grid
+resident in shared memory not at all).
 
 `stream`: the bandwidth a plain streaming kernel reaches for one colour
 sweep's transfer at N^3 -- three FP32 arrays of N^3/2 read, one written
@@ -63,7 +64,7 @@ def sor(n, iters, depth=0):
     it = s.diagnostics()["last_iterations"]
     per = t["sor_ms"] / max(1, it)
     print(f"sor n={n} sor_depth={depth}: {it} iterations, {per * 1e3:.1f} us per iteration, "
-          f"{6 * (n - 2) ** 3 / (per / 2 * 1e-3) / 1e9:.0f} GB/s algorithmic per sweep", flush=True)
+          f"{12 * (n - 2) ** 3 / (per * 1e-3) / 1e9:.0f} GB/s algorithmic", flush=True)
     s.close()
 
 

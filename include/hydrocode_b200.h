@@ -89,7 +89,11 @@ typedef struct hc_config {
     double omega;            /* SOR relaxation (default 1.5) */
     double tol;              /* SOR tolerance on max |phi_GS - phi_old| */
     int max_iter;
-    int sor_depth;           /* SOR kernels: 0 (default) colour-split sweeps;
+    int sor_depth;           /* SOR kernels, all with the same iterates:
+                                0 (default) many iterations per launch in
+                                shared memory where the grid fits, else two
+                                FP32 iterations per pass or FP64 colour-split
+                                sweeps;
                                 -3 colour-split with the FP32 correction
                                 sweeps staged by TMA where rows of one colour
                                 hold at most 256 cells, a multiple of 4;
