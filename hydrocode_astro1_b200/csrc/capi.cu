@@ -1275,8 +1275,9 @@ static HydroArgs hydro_args(hc_ctx *c)
     return a;
 }
 
-// One godunov step on the device state (no host synchronisation).
-static int step_once(hc_ctx *c, int *grav_status)
+// One godunov step on the device state (no host synchronisation); its dt goes
+// to *dt_host (pinned) as well.
+static int step_once(hc_ctx *c, int *grav_status, double *dt_host)
 {
     if (c->cfg.gravity_only) return set_err(HC_ERR_STATE, "gravity-only context has no hydro state");
     const bool f64 = c->cfg.precision == HC_FP64;
@@ -1297,6 +1298,7 @@ static int step_once(hc_ctx *c, int *grav_status)
         *grav_status = st;
     }
     HydroArgs a = hydro_args(c);
+    a.dt_host = dt_host;
     {
         FamTimer t(c, FAM_BC);
         CK(f64 ? fp64_dt(a, c->s) : fp32_dt(a, c->s));
@@ -1347,10 +1349,9 @@ extern "C" int hc_step(hc_ctx *c, int nsteps, double *dt_out)
     int worst = 0;
     for (int q = 0; q < nsteps; q++) {
         int gs = 1;
-        rc = step_once(c, &gs);
+        rc = step_once(c, &gs, c->hdt + q);
         if (rc) return rc;
         if (gs == -1) worst = -1;
-        CK(cudaMemcpyAsync(c->hdt + q, &c->sc->dt, sizeof(double), cudaMemcpyDeviceToHost, c->s));
     }
     if (c->cons_record && nsteps > 0) {
         rc = launch_cons_sums(c);
@@ -1382,9 +1383,8 @@ extern "C" int hc_step_host(hc_ctx *c, double *U, double *dt_out)
     else CK(fp32_from_aos64(c->stage, c->q32[c->cur], c->g.n, c->s));
     c->cfl_valid = 0;
     int gs = 1;
-    rc = step_once(c, &gs);
+    rc = step_once(c, &gs, c->hdt);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(c->hdt, &c->sc->dt, sizeof(double), cudaMemcpyDeviceToHost, c->s));
     if (c->cfg.precision == HC_FP64) CK(fp64_soa_to_aos(c->q64[c->cur], c->stage, c->g.n, c->s));
     else CK(fp32_to_aos64(c->q32[c->cur], c->stage, c->g.n, c->s));
     CK(cudaMemcpyAsync(U, c->stage, 5 * n * sizeof(double), cudaMemcpyDeviceToHost, c->s));

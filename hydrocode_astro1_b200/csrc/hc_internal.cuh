@@ -118,6 +118,7 @@ struct HydroArgs {
     const double *phig;     // potential used for g (last converged)
     DevScalars *sc;
     int step_parity;        // smax slot read = parity, written = parity^1
+    double *dt_host;        // the step's dt, in pinned host memory too
 };
 
 // FP64 (bit-exact) hydro path -- hydro_fp64.cu
