@@ -118,14 +118,20 @@ __device__ __forceinline__ void centre_of_mass(const Geom &g, const double *acc,
 // A guess only decides whether a record can be used; what is used is checked
 // against the sum itself.  The records hold for sums that keep their sign as
 // for those that return to zero in every row (z and the mixed moments of a
-// centred box), where the binade changes every few cells.
+// centred box), where the binade changes every few cells, and where symmetry
+// leaves rounding errors alone (a star without noise in a centred box, whole
+// solve of one iteration at 128^3: 35 ms cell by cell, 80 with the binade's
+// margins alone, 2.1 with those of exact additions).  Sums below 2^-963 are
+// taken cell by cell (1.4 to 4 times the one CTA's time).
 // Bound: a chain of dependent FP64 additions.  One CTA adding cell by cell (17
 // cycles a cell) took 4.65 ms at 64^3, 35.8 ms at 128^3 and 317 ms at 256^3 for both
 // passes; this takes 0.45-0.54, 1.3-1.8 and 7-17 ms, the last walk and, at
 // 256^3, the terms' arithmetic being the most of it.
 constexpr int SEQ_GRP = 32;        // runs of a group
-constexpr int SEQ_DIRECT = 14000;  // cells below which the sums are added cell by cell: 24^3 takes 230 us,
-                                   // the records' sixteen launches 225-265 us at 26^3
+constexpr int SEQ_RUN = 256;       // cells of a run, at most
+constexpr int SEQ_DIRECT = 20000;  // cells below which the sums are added cell by cell: a whole solve of one
+                                   // iteration takes 0.30 ms at 23^3 and 0.37 at 26^3, with the records'
+                                   // sixteen launches 0.35 to 0.55 ms on either
 constexpr double SEQ_ALL = 1e300;  // the margin before the first term
 
 struct SeqRecs {
@@ -141,18 +147,43 @@ struct SeqWork {
     int G;                      // cells of a run
 };
 
-// Partial sums: the sum, the largest unit and the least distance to a binade's end.
+// The margin of acc = was + t without rounding error (0 for others): acc is a
+// multiple of w, the lesser of its lowest bit and 2 U, and stays a double when
+// moved by a multiple of 2 U as long as it is below 2^53 w.  Out of line: few
+// additions need it.
+__device__ __noinline__ double seq_exact(double was, double t, double acc, int ue)
+{
+    const double bb = acc - was, err = (was - (acc - bb)) + (t - bb);
+    const int e = (__double2hiint(acc) >> 20) & 0x7ff;
+    if (err != 0.0 || ue <= 60 || ue >= 1900 || (e <= 110 && acc != 0.0)) return 0.0;
+    int w = ue - 51;   // biased exponent of 2 U
+    if (acc != 0.0) w = min(w, e - 53 + __ffsll((__double_as_longlong(acc) & ((1LL << 52) - 1)) | (1LL << 52)));
+    return __hiloint2double((w + 53) << 20, 0) - fabs(acc);
+}
+
+// Partial sums: the sum, the largest unit and the margin.
 struct SeqSum {
     double acc, margin;
     int ue;                     // biased exponent of the largest partial sum
+    template <bool MARGIN = true>
     __device__ __forceinline__ void add(double t)
     {
         if (t == 0.0) return;   // acc + 0 is acc
+        const double was = acc;
         acc += t;
         const int hi = __double2hiint(acc) & 0x7fffffff, e = hi >> 20;
+        if (!MARGIN) {
+            ue = max(ue, e);
+            return;
+        }
         const double m = fabs(acc), bin = __hiloint2double(e << 20, 0);
-        margin = fmin(margin, e > 60 && e < 2000 ? fmin(m - bin, 2.0 * bin - m) : 0.0);
+        double mi = e > 60 && e < 2000 ? fmin(m - bin, 2.0 * bin - m) : 0.0;
         ue = max(ue, e);
+        // only where the binade is so close that a start may well be past it
+        // (2^-22 of the largest partial sum): a random term's rounded sums
+        // hardly ever are
+        if (mi < margin && (__double2hiint(mi) >> 20) < ue - 22) mi = fmax(mi, seq_exact(was, t, acc, ue));
+        margin = fmin(margin, mi);
     }
 };
 __device__ __forceinline__ double seq_unit(int ue) { return __hiloint2double((ue - 52) << 20, 0); }
@@ -261,7 +292,7 @@ __global__ void __launch_bounds__(128) seq_first_kernel(GravArgs a, long long c0
     if (r >= n) return;
     const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
     SeqSum s = { w.pre[q * n + r], SEQ_ALL, 0 };
-    seq_cells<PASS>(a, q, c0 + r * w.G, w.G, c1, com, [&](double t) { s.add(t); });
+    seq_cells<PASS>(a, q, c0 + r * w.G, w.G, c1, com, [&](double t) { s.add<false>(t); });
     w.out1[0][q * n + r] = s.acc;
     w.ue1[0][q * n + r] = s.ue;
 }
@@ -328,23 +359,47 @@ struct SeqBatch {
     }
 };
 
-// A warp takes sum q over the runs [r0, r1), at most SEQ_GRP of them
-template <int PASS>
+// A warp takes sum q over the runs [r0, r1), at most SEQ_GRP of them, a run
+// whose record does not hold cell by cell: the terms of the run in parallel
+// into buf (SEQ_RUN doubles of the warp's own shared memory), then their chain.
+// TRACK: with the margin, for a record.
+template <int PASS, bool TRACK>
 __device__ __forceinline__ void seq_runs(const GravArgs &a, long long c0, long long c1, const SeqWork &w, int q,
-                                         long long r0, long long r1, const double *com, SeqSum &s)
+                                         long long r0, long long r1, const double *com, double *buf, SeqSum &s)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sjk = a.g.ny * a.g.nz;
     SeqBatch b;
     b.fetch(w.lev[0], PASS ? 9 : 4, q, r0 + lane);
     for (int j = 0; j < (int)(r1 - r0); j++) {
         if (b.use(j, s)) continue;
-        const long long c = c0 + (r0 + j) * w.G;
-        for (int x = 0; x < w.G; x += 32) {   // 32 terms at a time, then their chain
-            double t = 0.0;
-            seq_cells<PASS>(a, q, c + x + lane, 1, c1, com, [&](double v) { t = v; });
+        const long long c = c0 + (r0 + j) * w.G + lane, ce = min(c1, c - lane + w.G);
+        double r[SEQ_RUN / 32];
 #pragma unroll
-            for (int k = 0; k < 32; k++) s.add(__shfl_sync(0xffffffffu, t, k));
+        for (int u = 0; u < SEQ_RUN / 32; u++) r[u] = c + u * 32 < ce ? seq_density(a, c + u * 32) : 0.0;
+        int ci = (int)(c / sjk), rest = (int)(c % sjk), cj = rest / a.g.nz, ck = rest % a.g.nz;
+#pragma unroll
+        for (int u = 0; u < SEQ_RUN / 32; u++) {
+            if (u * 32 >= w.G) break;
+            buf[u * 32 + lane] = seq_term<PASS>(a, q, r[u], ci, cj, ck, com);
+            for (ck += 32; ck >= a.g.nz; ck -= a.g.nz)
+                if (++cj == a.g.ny) {
+                    cj = 0;
+                    ci++;
+                }
         }
+        __syncwarp();
+#pragma unroll 16
+        for (int k = 0; k < w.G; k += 2) {
+            const double2 v = *reinterpret_cast<const double2 *>(buf + k);
+            if (TRACK) {
+                s.add(v.x);
+                s.add(v.y);
+            } else {
+                s.acc += v.x;
+                s.acc += v.y;
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -354,6 +409,7 @@ template <int PASS>
 __global__ void __launch_bounds__(32) seq_groups_kernel(GravArgs a, long long c0, long long c1, SeqWork w,
                                                         const double *acc, int second)
 {
+    __shared__ __align__(16) double buf[SEQ_RUN];
     const int q = blockIdx.y, v = blockIdx.z;
     const long long h = blockIdx.x, n0 = w.lev[0].n, n = w.lev[1].n, r0 = h * SEQ_GRP;
     const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
@@ -361,7 +417,7 @@ __global__ void __launch_bounds__(32) seq_groups_kernel(GravArgs a, long long c0
     const double est = w.lev[0].g[q * n0 + r0];
     const double g = second ? seq_guess(w.out1[1], w.ue1[1][at], at, h, est, acc[q], v) : est;
     SeqSum s = { g, SEQ_ALL, 0 };
-    seq_runs<PASS>(a, c0, c1, w, q, r0, min(n0, r0 + SEQ_GRP), com, s);
+    seq_runs<PASS, true>(a, c0, c1, w, q, r0, min(n0, r0 + SEQ_GRP), com, buf, s);
     if (threadIdx.x != 0) return;
     if (!second) {
         w.out1[1][at] = s.acc;
@@ -429,7 +485,7 @@ template <int PASS>
 __global__ void __launch_bounds__(PASS ? 288 : 128) seq_walk_kernel(GravArgs a, long long c0, long long c1,
                                                                     SeqWork w, double *acc)
 {
-    __shared__ double term[(PASS ? 9 : 4) * SEQ_ST];
+    __shared__ __align__(16) double term[(PASS ? 9 : 4) * SEQ_ST];
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double com[3] = { a.sc->moments[1], a.sc->moments[2], a.sc->moments[3] };
     if (!w.G) {
@@ -445,7 +501,8 @@ __global__ void __launch_bounds__(PASS ? 288 : 128) seq_walk_kernel(GravArgs a, 
             const int j = (int)(h % 32);
             if (j == 0) b.fetch(w.lev[1], PASS ? 9 : 4, q, h + lane);
             if (!b.use(j, s))
-                seq_runs<PASS>(a, c0, c1, w, q, h * SEQ_GRP, min(w.lev[0].n, (h + 1) * SEQ_GRP), com, s);
+                seq_runs<PASS, false>(a, c0, c1, w, q, h * SEQ_GRP, min(w.lev[0].n, (h + 1) * SEQ_GRP), com,
+                                      term + q * SEQ_RUN, s);
         }
     }
     if (lane == 0) acc[q] = s.acc;
@@ -753,7 +810,7 @@ static SeqWork seq_layout(long long n0, void *buf, size_t *bytes)
 static SeqWork seq_work(long long n, void *buf)
 {
     int G = 32;
-    while (G < 256 && n / G > 4096) G *= 2;
+    while (G < SEQ_RUN && n / G > 4096) G *= 2;
     SeqWork w = seq_layout((n + G - 1) / G, buf, nullptr);
     w.G = G;
     return w;
@@ -761,9 +818,9 @@ static SeqWork seq_work(long long n, void *buf)
 
 size_t grav_seq_bytes(const Geom &g)
 {
-    // the most runs of any range of the grid: 4097 of fewer than 256 cells, or n / 256
+    // the most runs of any range of the grid: 4097 of fewer than SEQ_RUN cells, or n / SEQ_RUN
     size_t b = 0;
-    seq_layout(std::max<long long>(g.n / 256 + 1, std::min<long long>(g.n / 32 + 1, 4097)), nullptr, &b);
+    seq_layout(std::max<long long>(g.n / SEQ_RUN + 1, std::min<long long>(g.n / 32 + 1, 4097)), nullptr, &b);
     return b;
 }
 
