@@ -141,6 +141,7 @@ CAPI = {
                                     C.POINTER(C.c_float), C.c_int, C.c_int, C.POINTER(C.c_float)]),
     "hc_unet_wgrad_test": (C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_uint16), C.POINTER(C.c_uint16),
                                      C.c_int, C.POINTER(C.c_float)]),
+    "hc_resident_fault": (C.c_int, [C.c_void_p, C.c_int]),
     "hc_sor_solve_noalloc": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_double,
                                         C.c_double, C.c_double, C.c_double, C.c_double, C.c_int,
                                         C.c_double, C.c_void_p, C.POINTER(C.c_int), _dp]),

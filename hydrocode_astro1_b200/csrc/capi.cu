@@ -91,7 +91,8 @@ struct hc_ctx {
     float *e32, *r32, *e32b;     // mixed precision correction (ping-pong) / residual
     // resident sweeps (sor_resident.cuh): the grid's blocks, the message rows
     // and the number of the next launch's first sweep
-    int resident;                // 0 not looked at yet, 1 in use, -1 the grid does not fit
+    int resident;                // 0 not looked at yet, 1 in use, -1 the grid does not fit or a launch failed
+    int resident_fault;          // hc_resident_fault
     ResPlan rplan;
     void *exch;
     unsigned epoch;
@@ -631,8 +632,14 @@ static bool resident_sweeps(hc_ctx *c, size_t elem)
         c->resident = -1;
         if (grav_resident_plan(c->g, elem, &c->rplan)) {
             void *p = nullptr;
-            if (cudaMalloc(&p, c->rplan.exch_bytes) != cudaSuccess) {
+            // FP64: the new boundary values, beside the potential that a solve
+            // taken again starts from
+            if (cudaMalloc(&p, c->rplan.exch_bytes) != cudaSuccess ||
+                (elem == 8 && !c->phi2 &&
+                 cudaMalloc((void **)&c->phi2, (size_t)c->g.n * sizeof(double)) != cudaSuccess)) {
                 (void)cudaGetLastError();   // no room: the separate sweeps need none
+                cudaFree(p);
+                c->phi2 = nullptr;
             } else if (cudaMemsetAsync(p, 0, c->rplan.exch_bytes, c->s) != cudaSuccess) {
                 cudaFree(p);
             } else {
@@ -643,6 +650,45 @@ static bool resident_sweeps(hc_ctx *c, size_t elem)
         }
     }
     return c->resident == 1;
+}
+
+// One resident launch of n iterations: false where it was refused; and whether
+// it gave up (hsc->lost, copied with the stop flag).  It needs all its blocks on
+// the GPU at once, and a block waits a limited time for another, so it can fail
+// where the separate sweeps do not (a GPU shared with other work): they take
+// the solve again from its start, and every later one of the context.
+template <typename F>
+static bool resident_launch(hc_ctx *c, int n, F launch)
+{
+    ResPlan p = c->rplan;
+    if (c->resident_fault == 2) {
+        p.absent = 1;
+        p.wait_ns = 1000000;
+    }
+    const cudaError_t e = c->resident_fault == 1 ? cudaErrorCooperativeLaunchTooLarge : launch(p, c->epoch);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();   // an error that stays comes back at the next launch
+        c->resident = -1;
+        if (c->debug) fprintf(stderr, "[hc] resident sweeps refused (%s): separate sweeps\n", cudaGetErrorString(e));
+        return false;
+    }
+    c->epoch += 4u * (unsigned)n + 16u;
+    c->sor_launches += 1;
+    return true;
+}
+static bool resident_lost(hc_ctx *c)
+{
+    if (!c->hsc->lost) return false;
+    c->resident = -1;
+    if (c->debug) fprintf(stderr, "[hc] resident sweeps gave up waiting: separate sweeps\n");
+    return true;
+}
+
+extern "C" int hc_resident_fault(hc_ctx *c, int kind)
+{
+    if (!c || kind < 0 || kind > 2) return set_err(HC_ERR_ARG, "bad argument");
+    c->resident_fault = kind;
+    return HC_OK;
 }
 
 // Whether an FP32 context's sweeps run as streaming passes (where they do not
@@ -707,8 +753,6 @@ static int sor_fp64(hc_ctx *c, const double *rho)
     int rc = ensure_res(c, a.max_iter);
     if (rc) return rc;
     a.res = c->res;
-    CK(cudaMemsetAsync(&c->sc->done, 0, 2 * sizeof(int), c->s));    // done, last_iter
-    CK(grav_reset_slots(a, 0, std::max(a.max_iter, 1), c->s));
     rc = grav_moments(c, a);
     if (rc) return rc;
     if (a.max_iter <= 0) {
@@ -722,7 +766,6 @@ static int sor_fp64(hc_ctx *c, const double *rho)
     // place between phi (buf 0) and phi2 (buf 1): iteration t reads buf[t%2],
     // writes buf[(t+1)%2].  All three give the same iterates.
     const bool split = c->cfg.sor_depth == 0 && c->g.nz >= 3;
-    const bool resident = split && resident_sweeps(c, sizeof(double));
     const bool wave = c->cfg.sor_depth >= 1 && c->g.nz >= 3;
     double *buf[2] = { c->phi, c->phi2 };
     if (split) {
@@ -730,8 +773,6 @@ static int sor_fp64(hc_ctx *c, const double *rho)
         if (!c->phs) rc = dmalloc((void **)&c->phs, ns * sizeof(double));
         if (!rc && !c->rhs) rc = dmalloc((void **)&c->rhs, ns * sizeof(double));
         if (rc) return rc;
-        CK(grav_split_fields(a, c->phs, c->rhs, c->s));
-        c->launches += 2;
     }
     if (wave) {
         if (!c->phi2) {
@@ -760,57 +801,79 @@ static int sor_fp64(hc_ctx *c, const double *rho)
         }
         return HC_OK;
     };
-    {
-        FamTimer t(c, FAM_SOR);
-        rc = one_iter(0);
-        if (rc) return rc;
-    }
-    // the first iteration swept with the previous boundary; now the new one
-    if (wave) {
-        GravArgs b = a;
-        b.phi = buf[1];
-        rc = grav_boundary_values(c, b);
-        if (rc) return rc;
-    }
-    rc = grav_boundary_values(c, a);
-    if (rc) return rc;
-    if (split) {
-        CK(grav_split_boundary(a, c->phs, c->s));
-        c->launches += 1;
-    }
-    int it = 1, done = 0, last = 0;
-    // a resident launch stops by itself: no polls in between, the cap only
-    // bounds one launch's duration
-    int batch = resident ? 4096 : 16;
-    while (true) {
-        int end = std::min(a.max_iter, it + batch);
+    int done = 0, last = 0;
+    // once; again with the separate sweeps where a resident launch failed
+    // (phi is still the solve's start then, its faces included)
+    for (bool finished = false; !finished;) {
+        const bool resident = split && resident_sweeps(c, sizeof(double));
+        CK(cudaMemsetAsync(&c->sc->done, 0, 3 * sizeof(int), c->s));    // done, last_iter, lost
+        CK(grav_reset_slots(a, 0, std::max(a.max_iter, 1), c->s));
+        if (split) {
+            CK(grav_split_fields(a, c->phs, c->rhs, c->s));
+            c->launches += 2;
+        }
         {
             FamTimer t(c, FAM_SOR);
-            if (resident && end > it) {
-                CK(grav_sor_resident(a, c->phs, c->rhs, c->rplan, c->exch, c->epoch, it, end - it, c->s));
-                c->epoch += 4u * (unsigned)(end - it) + 16u;
-                c->sor_launches += 1;
-            } else {
-                for (int q = it; q < end; q++) {
-                    rc = one_iter(q);
-                    if (rc) return rc;
-                }
-                CK(grav_check(a, end, c->s));
-            }
+            rc = one_iter(0);
+            if (rc) return rc;
         }
-        c->launches += 1;
-        CK(cudaMemcpyAsync(&c->hsc->done, &c->sc->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->s));
-        const int nb = std::min(end - it, 512);
-        if (!c->hslots && cudaMallocHost((void **)&c->hslots, 512 * sizeof(double)) != cudaSuccess)
-            return set_err(HC_ERR_NOMEM, "pinned slot buffer");
-        CK(cudaMemcpyAsync(c->hslots, c->res + (end - nb), nb * sizeof(double), cudaMemcpyDeviceToHost, c->s));
-        rc = sync_ctx(c);
+        // the first iteration swept with the previous boundary; now the new one
+        GravArgs b = a;
+        if (wave) {
+            b.phi = buf[1];
+            rc = grav_boundary_values(c, b);
+            if (rc) return rc;
+            b.phi = a.phi;
+        }
+        if (resident && a.grav_bc != 2) {
+            b.phi = c->phi2;
+            if (a.grav_bc == 0)   // periodic faces are copies of faces
+                CK(cudaMemcpyAsync(b.phi, c->phi, (size_t)c->g.n * sizeof(double), cudaMemcpyDeviceToDevice, c->s));
+        }
+        rc = grav_boundary_values(c, b);
         if (rc) return rc;
-        done = c->hsc->done;
-        last = c->hsc->last_iter;
-        if (done || end >= a.max_iter) break;
-        it = end;
-        if (!resident) batch = next_batch(c->hslots, nb, a.tol, batch);
+        if (split) {
+            CK(grav_split_boundary(b, c->phs, c->s));
+            c->launches += 1;
+        }
+        // a resident launch stops by itself: no polls in between, the cap only
+        // bounds one launch's duration
+        int it = 1, batch = resident ? 4096 : 16;
+        while (true) {
+            int end = std::min(a.max_iter, it + batch);
+            {
+                FamTimer t(c, FAM_SOR);
+                if (resident && end > it) {
+                    if (!resident_launch(c, end - it, [&](const ResPlan &p, unsigned epoch) {
+                            return grav_sor_resident(a, c->phs, c->rhs, p, c->exch, epoch, it, end - it, c->s);
+                        }))
+                        break;
+                } else {
+                    for (int q = it; q < end; q++) {
+                        rc = one_iter(q);
+                        if (rc) return rc;
+                    }
+                    CK(grav_check(a, end, c->s));
+                }
+            }
+            c->launches += 1;
+            CK(cudaMemcpyAsync(&c->hsc->done, &c->sc->done, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->s));
+            const int nb = std::min(end - it, 512);
+            if (!c->hslots && cudaMallocHost((void **)&c->hslots, 512 * sizeof(double)) != cudaSuccess)
+                return set_err(HC_ERR_NOMEM, "pinned slot buffer");
+            CK(cudaMemcpyAsync(c->hslots, c->res + (end - nb), nb * sizeof(double), cudaMemcpyDeviceToHost, c->s));
+            rc = sync_ctx(c);
+            if (rc) return rc;
+            if (resident && resident_lost(c)) break;
+            done = c->hsc->done;
+            last = c->hsc->last_iter;
+            if (done || end >= a.max_iter) {
+                finished = true;
+                break;
+            }
+            it = end;
+            if (!resident) batch = next_batch(c->hslots, nb, a.tol, batch);
+        }
     }
     int used = done ? last : a.max_iter;
     if (wave && (used & 1)) std::swap(c->phi, c->phi2);   // result in buf[used % 2]
@@ -847,8 +910,8 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
     // one in-place kernel per colour on the natural layout; >= 1: wavefront
     // passes of that many FP32 iterations per HBM pass on the natural layout
     const bool split = (c->cfg.sor_depth == 0 || c->cfg.sor_depth == -2 || c->cfg.sor_depth == -3) && c->g.nz >= 3;
-    const bool resident = split && resident_sweeps(c, sizeof(float));
-    const bool stream = split && !resident && stream_sweeps(c);
+    bool resident = split && resident_sweeps(c, sizeof(float));
+    bool stream = split && !resident && stream_sweeps(c);
     const bool wave2 = split && c->cfg.sor_depth == -2 && mixed_wave_split_ok(c->g);
     const int depth = wave2 ? 2 : (split ? -1 : c->cfg.sor_depth);
     int rc = ensure_res(c, a.max_iter);
@@ -956,7 +1019,7 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
         const double tol_last = a.tol * HC_LAST_CYCLE_TARGET;
         const double thresh = std::max(tol_last, HC_CYCLE_REDUCTION * dmax);
         const int budget = a.max_iter - total;
-        CK(cudaMemsetAsync(&c->sc->done, 0, 2 * sizeof(int), c->s));
+        CK(cudaMemsetAsync(&c->sc->done, 0, 3 * sizeof(int), c->s));
         CK(grav_reset_slots(a, 0, budget + 8, c->s));
         float *eb[2] = { c->e32, c->e32b };
         // the passes write every interior cell of their output; its boundary
@@ -971,15 +1034,31 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
         double best = 1e300;
         if (!c->hslots && cudaMallocHost((void **)&c->hslots, 512 * sizeof(double)) != cudaSuccess)
             return set_err(HC_ERR_NOMEM, "pinned slot buffer");
+        // a resident launch failed: the cycle again from its start, e = 0
+        auto without_resident = [&]() -> int {
+            resident = false;
+            stream = stream_sweeps(c);
+            CK(cudaMemsetAsync(c->e32, 0, (size_t)split_len(c->g) * sizeof(float), c->s));
+            CK(cudaMemsetAsync(&c->sc->done, 0, 3 * sizeof(int), c->s));
+            CK(grav_reset_slots(a, 0, budget + 8, c->s));
+            it = best_it = 0;
+            batch = 16;
+            best = 1e300;
+            return HC_OK;
+        };
         while (true) {
             int end = std::min(budget, it + batch);
             {
                 FamTimer t(c, FAM_SOR);
                 if (resident) {
-                    CK(mixed_sor32_resident(a, c->e32, c->r32, c->rplan, c->exch, c->epoch, it, end - it, thresh,
-                                            c->s));
-                    c->epoch += 4u * (unsigned)(end - it) + 16u;
-                    c->sor_launches += 1;
+                    if (!resident_launch(c, end - it, [&](const ResPlan &p, unsigned epoch) {
+                            return mixed_sor32_resident(a, c->e32, c->r32, p, c->exch, epoch, it, end - it, thresh,
+                                                        c->s);
+                        })) {
+                        rc = without_resident();
+                        if (rc) return rc;
+                        continue;
+                    }
                 } else if (stream) {
                     rc = stream_batch(c, run, it, end, pass);
                     if (rc) return rc;
@@ -1020,11 +1099,16 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
                 c->launches += 1;
             }
             processed = end;
-            CK(cudaMemcpyAsync(&c->hsc->done, &c->sc->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->s));
+            CK(cudaMemcpyAsync(&c->hsc->done, &c->sc->done, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->s));
             const int nb = std::min(end - it, 512);
             CK(cudaMemcpyAsync(c->hslots, c->res + (end - nb), nb * sizeof(double), cudaMemcpyDeviceToHost, c->s));
             rc = sync_ctx(c);
             if (rc) return rc;
+            if (resident && resident_lost(c)) {
+                rc = without_resident();
+                if (rc) return rc;
+                continue;
+            }
             done = c->hsc->done;
             last = c->hsc->last_iter;
             if (stream) {

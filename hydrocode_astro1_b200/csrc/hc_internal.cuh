@@ -60,7 +60,7 @@ struct DevScalars {
     double dt;                    // current step dt
     int done;                     // SOR converged / stopped flag
     int last_iter;                // iterations of the finished solve
-    int overshoot;                // temporal blocking passed tol inside a pass
+    int lost;                     // a resident launch gave up: the solve is taken again by the separate sweeps
     int err;                      // sticky device error code
     unsigned long long resid_bits; // scratch
     double moments[4 + 9];        // M, COM, Q (reference mode)
@@ -249,7 +249,12 @@ cudaError_t grav_sor_split(const GravArgs &a, double *phs, const double *rhs, in
 // it does not fit), and iterations it0 .. it0 + n - 1 until the stop test
 // (the launch sets done / last_iter).  exch: plan.exch_bytes of device memory,
 // zeroed once and kept; epoch: a number that advances by 4 n + 16 per launch
+// (plan.wait_ns: the longest wait for another block, after which the launch
+// sets sc->lost and ends; plan.absent: blocks that the meetings wait for in
+// vain, for tests)
 struct ResPlan {
+    unsigned long long wait_ns = 4000000000ULL;
+    unsigned absent = 0;
     int gi = 0, gj = 0, BI = 0, BJ = 0, Hp = 0;
     size_t smem = 0, exch_bytes = 0;
 };

@@ -21,8 +21,8 @@
 // Messages carry their own flags: every 8-byte word is {32 bits of payload,
 // sweep number}, stored and loaded as one relaxed 64-bit access, so a row
 // needs no fence, no flag line and no second round trip.  A receiver polls
-// the words it needs (bounded; on a timeout the kernel sets sc->err and
-// leaves).  One buffer per colour is enough: a sender overwrites its colour's
+// the words it needs (bounded; on a timeout the kernel sets sc->lost and
+// leaves, and the caller takes the solve again by the separate sweeps).  One buffer per colour is enough: a sender overwrites its colour's
 // rows two sweeps later, after the receiver's rows of the sweep between,
 // which the receiver sends after it has read the older ones.
 //
@@ -52,7 +52,6 @@ namespace hc {
 constexpr int RS_NT = 512;                    // threads of a CTA
 constexpr int RS_NW = RS_NT / 32;
 constexpr int RS_MAXGROUP = 128;              // iterations between two meetings
-constexpr unsigned long long RS_WAIT_NS = 4000000000ULL;
 constexpr int RS_TASKS = 1024;                // warp tasks of a half sweep, at most
 constexpr int RS_STATIC = 3072;               // room for the kernel's static shared memory
 constexpr size_t RES_EXCH_HEAD = 256;         // arrival counter, before the message rows
@@ -72,6 +71,8 @@ struct ResArgs {
     DevScalars *sc;
     unsigned magic;            // ceil(2^32 / vectors per row), 0 for one
     unsigned epoch;            // sweep numbers used: epoch .. epoch + 4 n + 16
+    unsigned absent;           // blocks that no meeting sees
+    unsigned long long wait_ns;
 };
 
 __device__ __forceinline__ unsigned long long rs_word(unsigned v, unsigned flag)
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     };
     auto give_up = [&]() {
         quit = 1;
-        atomicExch(&A.sc->err, HC_ERR_TIMEOUT);
+        atomicExch(&A.sc->lost, 1);
     };
     // colour o's rows around the block, as sweep `flag` left them
     auto receive = [&](int o, unsigned flag) {
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
                     if ((++tries & 1023u) == 0) {
                         const unsigned long long now = rs_now();
                         if (!t0) t0 = now;
-                        if (now - t0 > RS_WAIT_NS || *(volatile int *)&A.sc->err) {
+                        if (now - t0 > A.wait_ns || *(volatile int *)&A.sc->lost) {
                             give_up();
                             break;
                         }
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
             hit = 1 << 30;
             __threadfence();
             atomicAdd(A.meet, 1u);
-            const unsigned want = (unsigned)met * (unsigned)ncta;
+            const unsigned want = (unsigned)met * (unsigned)ncta + A.absent;
             unsigned seen, tries = 0;
             unsigned long long w0 = 0;
             while (true) {
@@ -614,7 +615,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
                 if ((++tries & 1023u) == 0) {
                     const unsigned long long now = rs_now();
                     if (!w0) w0 = now;
-                    if (now - w0 > RS_WAIT_NS || *(volatile int *)&A.sc->err) {
+                    if (now - w0 > A.wait_ns || *(volatile int *)&A.sc->lost) {
                         give_up();
                         break;
                     }
@@ -743,6 +744,8 @@ cudaError_t run_resident(const ResPlan &p, T *e, const T *src, const Split &sp, 
     a.sc = sc;
     a.magic = (unsigned)((0x100000000ULL + (unsigned)(p.Hp / Pack<T>::V) - 1) / (unsigned)(p.Hp / Pack<T>::V));
     a.epoch = epoch;
+    a.absent = p.absent;
+    a.wait_ns = p.wait_ns;
     const bool al = sp.H % Pack<T>::V == 0 && ((uintptr_t)e | (uintptr_t)src) % 16 == 0 && sp.cs % Pack<T>::V == 0;
     if (!al) return launch_resident<T, false, false>(a, p.smem, s);
     return sp.nz % 2 == 0 ? launch_resident<T, true, true>(a, p.smem, s) : launch_resident<T, true, false>(a, p.smem, s);

@@ -336,6 +336,13 @@ int hc_unet_conv_test(int nx, int ny, int nz, const uint16_t *x, const uint16_t 
                       int out_mode, int act, float *out);
 int hc_unet_wgrad_test(int nx, int ny, int nz, const uint16_t *x, const uint16_t *dy, int max_parts, float *dw);
 
+/* Makes the context's next resident relaxation launch (sor_depth 0) fail, for
+ * tests of what follows: kind 1 as if the launch had been refused, 2 by a wait
+ * for a block that does not exist (given up after a millisecond), 0 not at
+ * all.  The solve is then taken again by the separate sweeps, with the same
+ * result, and so is every later one of the context. */
+int hc_resident_fault(hc_ctx *ctx, int kind);
+
 /* Red-black SOR to tolerance on caller-owned DEVICE arrays, allocating
  * nothing.  No counterpart in the reference: it exists for callers that own
  * all device memory themselves (a fixed arena reserved at start-up, a pool
