@@ -32,8 +32,12 @@
 // group all CTAs meet, read the norms of its iterations, and either write
 // their block back (the next group's starting point) or, when an iteration
 // inside the group was the last, reload the group's start and run exactly the
-// iterations up to it again.  Group lengths follow the norms' rate, so the
-// last groups are short.  One CTA alone tests after every iteration.
+// iterations up to it again.  The first group has four, the next ones at most
+// twice as many as the one before, and where few are left by the norms' rate just
+// those: a meeting costs half an iteration (64^3) to three (150^3), a group that
+// is too long its iterations twice.  (First groups of 16 made solves of 2 to 14
+// iterations slower than the separate sweeps; a solve of 3 at 64^3 in FP64 took
+// 298 us against 226, now 222; one of 12 350, 266 and 265.)  One CTA alone tests after every iteration.
 //
 // Per cell the update is SorCoef<T>::update with the operands of the other
 // sweep kernels, and the cells of a colour are independent: the iterates, the
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     using Row = ResRow<T, AL>;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     __shared__ unsigned long long bmax[2];
-    __shared__ int quit, hit, glen;
+    __shared__ int quit, hit, glen, met;
     __shared__ double gv[2];
     __shared__ unsigned short tasks[RS_TASKS];
 
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
         return;
     }
     if (tid == 0) {
-        quit = 0;
+        quit = met = 0;
         bmax[0] = bmax[1] = 0;
     }
 
@@ -458,9 +462,9 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     __syncthreads();
     unsigned ep = A.epoch;   // number of the last sweep sent
     if (multi) send_edges(1, ep);
-    int t = A.it0, met = 0;
+    int t = A.it0;
     const int tend = A.it0 + A.n;
-    int len = multi ? min(16, A.n) : 1;
+    int len = multi ? min(4, A.n) : 1;
     int t0 = t, t1 = min(tend, t + len);   // the group of iterations
     int last = -1;                         // the iteration that converged
     bool again = false;                    // the group runs again, up to `last`
@@ -601,9 +605,9 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
             continue;
         }
         // all CTAs have recorded the norms of their iterations so far
-        met++;
         if (tid == 0) {
             hit = 1 << 30;
+            met++;
             __threadfence();
             atomicAdd(A.meet, 1u);
             const unsigned want = (unsigned)met * (unsigned)ncta + A.absent;
@@ -644,13 +648,14 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
         }
         if (last >= 0 || t >= tend) break;
         if (tid == 0) {
-            // iterations left at the norms' rate; 80% of them in the next group
+            // iterations left at the norms' rate over the last ones of the group,
+            // seven tenths of them while they are many
             const int w = min(32, t1 - t0 - 1);
             int l = min(2 * len, RS_MAXGROUP);
-            if (w >= 3 && gv[1] > 0.0 && gv[0] > gv[1]) {
+            if (w >= 1 && gv[1] > 0.0 && gv[0] > gv[1]) {
                 const float rate = __logf((float)(gv[0] / gv[1])) / (float)w;
                 const float left = __logf((float)(gv[1] / A.thresh)) / rate;
-                l = left < 5.f ? 4 : (left * 0.8f < (float)RS_MAXGROUP ? (int)(left * 0.8f) : RS_MAXGROUP);
+                l = min(l, left < 10.f ? max(1, (int)left) : (int)fminf(left * 0.7f, (float)RS_MAXGROUP));
             }
             glen = l;
         }

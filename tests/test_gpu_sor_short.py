@@ -1,0 +1,65 @@
+"""Resident solves of few iterations: they end after exactly the iteration whose
+norm is below the tolerance, whatever group it falls into, and take no longer
+than the separate sweeps."""
+import time
+
+import numpy as np
+import pytest
+
+import hydrocode_astro1_b200 as hc
+
+pytestmark = pytest.mark.gpu
+
+
+def start(shape):
+    x = np.meshgrid(*[(np.arange(n) + 0.5) / n - 0.5 for n in shape], indexing="ij", sparse=True)
+    return np.maximum(1e-6, 1 - 8 * sum(v * v for v in x)) + 0 * x[0]
+
+
+@pytest.mark.parametrize("precision", [hc.FP64, hc.FP32])
+def test_every_stopping_iteration(precision):
+    shape = (40, 36, 48)
+    q = np.zeros((5,) + shape)
+    q[0], q[4] = start(shape), 1.0
+    phi0 = np.random.default_rng(0).standard_normal(shape)
+    with hc.HydroSolver3D(shape, G=1.0, precision=precision, moment_order=hc.MOMENTS_TREE) as s:
+        s.set_state(q)
+
+        def solve(max_iter, tol):
+            s.set_gravity_params(1.5, max_iter, tol)
+            s.set_phi(phi0)
+            s.gravity_solve()
+            d = s.diagnostics()
+            return s.phi(), d["last_iterations"], d["last_residual"]
+
+        for k in range(1, 41):
+            want = solve(k, 1e-30)
+            assert want[1] == k
+            if precision == hc.FP64:   # the mixed solve's norms go through its cycles
+                got = solve(1000, want[2] * (1 + 1e-12))
+                assert got[1:] == want[1:] and np.array_equal(got[0], want[0])
+
+
+@pytest.mark.parametrize("eps", [3e-5, 1e-4])
+def test_short_solves_take_no_longer(eps):
+    shape = (64, 64, 64)
+    rho = start(shape)
+    changed = rho * (1 + eps * np.random.default_rng(0).random(shape))
+
+    def best(fault):
+        with hc.HydroSolver3D(shape, G=1.0, gravity_only=1, max_iter=20000, tol=1e-6,
+                              moment_order=hc.MOMENTS_TREE) as s:
+            hc.lib().hc_resident_fault(s.h, fault)
+            s.gravity_solve(rho)
+            s.gravity_solve(rho)
+            phi, times = s.phi(), []
+            for _ in range(20):
+                s.set_phi(phi)
+                t = time.perf_counter()
+                s.gravity_solve(changed)
+                times.append(time.perf_counter() - t)
+                assert 2 <= s.diagnostics()["last_iterations"] <= 15
+            return min(times)
+
+    resident, separate = best(0), best(1)
+    assert resident < 1.1 * separate, (resident, separate)
