@@ -672,6 +672,31 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     }
 }
 
+// Whether the plan beats the separate sweeps.  Blocks of a few long rows are
+// mostly edge: every iteration polls and posts them all, 512 vectors a round, and
+// that takes longer than the sweeps (us an iteration, sweeps and resident:
+// FP64 4x15x4132 5.9 and 23.5, 20x20x1000 8.1 and 12.0, 64x64x600 18.6 and 25.3,
+// 118x3x1059 9.4 and 6.3; FP32 23x10x5511 9.3 and 24.9, 8x8x512 5.8 and 4.8).  Both
+// times by fits to 270 shapes, good to 15%: rounds and warp units of a half sweep;
+// cells, with the sweeps' idle lanes.  Blocks with fewer edge rows, or rows
+// below 48 vectors, are always faster resident.
+inline bool res_pays(const ResPlan &p, const Geom &g, size_t elem)
+{
+    const int V = (int)(16 / elem), Hv = p.Hp / V, H = (g.nz + 1) / 2;
+    if (Hv < 48 || p.BI * p.BJ > 3 * (p.BI + p.BJ)) return true;
+    const int edge = (p.gi > 1 ? 2 : 1) * p.BJ + (p.gj > 1 ? 2 : 1) * p.BI;   // a face's rows count half
+    const int rounds = (edge * Hv + RS_NT - 1) / RS_NT, chunks = ((p.BJ + 1) / 2 * Hv + 31) / 32;
+    int units = 1 << 30;
+    for (int t = 1; t <= std::min(p.BI, 8); t++)
+        if (chunks * t <= RS_TASKS)
+            units = std::min(units, (chunks * t + RS_NW - 1) / RS_NW * ((p.BI + t - 1) / t + 2));
+    const double res = p.gi * p.gj > 1 ? 1.38 * rounds + 1.83 * units - 1.75 : 1.85 * rounds + 0.62 * units + 0.36;
+    const int lanes = elem == 4 && H % V == 0 ? 32 * V : 32;
+    const double mcell = 1e-6 * (double)g.n / H * ((H + lanes - 1) / lanes * lanes);
+    const double sweeps = elem == 8 ? 5.1 + 5.4 * mcell : 5.9 + (lanes > 32 ? 2.0 : 2.77) * mcell;
+    return res <= sweeps;
+}
+
 // Blocks of a grid (ResPlan): the split into gi x gj CTAs (at most one per SM) with the
 // least work per CTA that fits shared memory; one CTA alone when its work is
 // below the cost of the exchange (about 300 vectors).
@@ -702,7 +727,7 @@ inline bool res_plan(const Geom &g, size_t elem, int sms, size_t smem_max, ResPl
             }
         }
     }
-    if (best >= 1e300) return false;
+    if (best >= 1e300 || !res_pays(p, g, elem)) return false;
     *out = p;
     return true;
 }
