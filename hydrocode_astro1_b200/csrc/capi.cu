@@ -91,13 +91,13 @@ struct hc_ctx {
     float *e32, *r32, *e32b;     // mixed precision correction (ping-pong) / residual
     // resident sweeps (sor_resident.cuh): the grid's blocks, the message rows
     // and the number of the next launch's first sweep
-    int resident;                // 0 not looked at yet, 1 in use, -1 the grid does not fit or a launch failed
+    int resident;                // 0 not looked at yet, 1 in use, -1 not for this grid, or a launch failed
     int resident_fault;          // hc_resident_fault
     ResPlan rplan;
     void *exch;
     unsigned epoch;
     // streaming passes (sor_stream.cuh) of grids that do not fit
-    int stream;                  // 0 not looked at yet, 1 in use, -1 the layout does not allow them
+    int stream;                  // 0 not looked at yet, 1 in use, -1 not for this grid
     StreamTile tile[2];          // passes of 1 and of 2 iterations
     double *gx, *gy, *gz;
     double *res;

@@ -810,7 +810,8 @@ bool mixed_stream_tile(const Geom &g, int its, StreamTile *out)
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return false;
-    return stream_tile(make_split(g), its, sms, out);
+    const Split sp = make_split(g);
+    return stream_tile(sp, its, sms, out) && (its != 2 || stream_pays(*out, sp, sms));
 }
 
 cudaError_t mixed_stream_check(const GravArgs &a, int iter0, int pair, double thresh, cudaStream_t s)

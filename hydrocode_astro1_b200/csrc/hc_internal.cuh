@@ -267,6 +267,7 @@ struct StreamTile {
     int tj, tk, L, ch;     // tiles along j and k, planes of a chunk, chunks
     unsigned magic;        // ceil(2^32 / WV), 0 for one
 };
+// false: the layout does not allow them, or the separate sweeps are faster
 bool mixed_stream_tile(const Geom &g, int its, StreamTile *out);
 // iterations iter0 .. iter0 + its - 1 unless one of the `pair` before them
 // ended the solve (force: whatever they say); the check after the last pass

@@ -285,6 +285,23 @@ inline bool stream_tile(const Split &sp, int its, int sms, StreamTile *out)
     return true;
 }
 
+// Whether passes of two iterations over tiles t beat the separate sweeps.  A
+// grid of few planes or rows, or of rows that leave few windows, is mostly halo
+// (us an iteration, sweeps and passes: 6x1132x2048 28.3 and 56.2, 2119x9x512 32.4
+// and 75.6, 24x946x512 31.3 and 40.6; 24x5016x128 69.8 and 39.9, 1928x40x128 47.3
+// and 33.5).  Both times by fits to 206 shapes, good to 12%: the steps of the
+// waves, those that update planes, their warps; the cells of inner planes, the
+// sweeps' idle lanes and rows.
+inline bool stream_pays(const StreamTile &t, const Split &sp, int sms)
+{
+    const int waves = (t.tj * t.tk * t.ch + sms - 1) / sms, steps = (t.L + 6 + 5) / 6 * 6 + 2;
+    const int act = t.ch == 1 ? t.L : steps, warps = (t.W * t.WV + 31) / 32;
+    const double passes = 0.33 + waves * (0.117 * steps + 0.438 * act + 0.0126 * steps * warps);
+    const double lanes = (double)((sp.H + 127) / 128 * 128) / sp.H, rows = (double)((sp.ny + 7) / 8 * 8) / sp.ny;
+    const double mcell = 1e-6 * (sp.nx - 2) * sp.ny * sp.nz;
+    return passes <= 5.65 + mcell * (0.385 + 2.095 * lanes + 0.80 * (rows - 1.0));
+}
+
 template <int NH, int NT, bool EVEN>
 cudaError_t launch_stream(const StreamArgs &a, cudaStream_t s)
 {
