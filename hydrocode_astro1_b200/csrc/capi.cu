@@ -520,11 +520,11 @@ extern "C" int hc_get_state_soa(hc_ctx *c, double *q)
 }
 
 // ---------------------------------------------------------------- gravity
-// Work of the sequential moments, once per context; without room for it they
-// are added cell by cell.
+// Work of the sequential moments, once per context; without room for it, and
+// on small grids, they are added cell by cell.
 static void *ensure_seq(hc_ctx *c)
 {
-    if (!c->seq && !c->seq_tried) {
+    if (!c->seq && !c->seq_tried && grav_seq_records(c->g.n)) {
         c->seq_tried = 1;
         if (cudaMalloc(&c->seq, grav_seq_bytes(c->g)) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -587,8 +587,7 @@ static int grav_moments(hc_ctx *c, const GravArgs &a0)
     FamTimer t(c, FAM_MOM);
     if (a.lmax == 0) {
         if (a.moment_order == HC_MOMENTS_SEQUENTIAL && a.rho) {
-            CK(grav_moments_sequential(a, c->s));
-            c->launches += a.seq ? 16 : 4;
+            CK(grav_moments_sequential(a, c->s, &c->launches));
         } else {
             CK(grav_moments_tree(a, c->s));
             c->launches += 4;
@@ -1755,13 +1754,14 @@ extern "C" int hc_slab_moments(hc_ctx *c, int pass, double *buf)
         if (slab_sequential(c)) {
             CK(cudaMemcpyAsync(c->slab_buf, buf, count * sizeof(double), cudaMemcpyHostToDevice, c->s));
             a.seq = ensure_seq(c);
-            CK(grav_moments_seq_slab(a, pass, c->slab_buf, c->s));
+            CK(grav_moments_seq_slab(a, pass, c->slab_buf, c->s, &c->launches));
         } else if (c->cfg.lmax == 0) {
             CK(grav_moments_tree_parts(a, pass, c->slab_buf, c->s));
+            c->launches += 1;
         } else {
             CK(grav_moments_lmax_parts(a, pass, c->slab_buf, c->s));
+            c->launches += 1;
         }
-        c->launches += 1;
     }
     CK(cudaMemcpyAsync(buf, c->slab_buf, count * sizeof(double), cudaMemcpyDeviceToHost, c->s));
     return sync_ctx(c);

@@ -816,6 +816,8 @@ static SeqWork seq_work(long long n, void *buf)
     return w;
 }
 
+bool grav_seq_records(long long cells) { return cells >= SEQ_DIRECT; }
+
 size_t grav_seq_bytes(const Geom &g)
 {
     // the most runs of any range of the grid: 4097 of fewer than SEQ_RUN cells, or n / SEQ_RUN
@@ -825,11 +827,14 @@ size_t grav_seq_bytes(const Geom &g)
 }
 
 template <int PASS>
-static cudaError_t seq_run(const GravArgs &a, long long c0, long long c1, double *acc, cudaStream_t s)
+static cudaError_t seq_run(const GravArgs &a, long long c0, long long c1, double *acc, cudaStream_t s,
+                           long long *launched)
 {
     constexpr int NV = PASS ? 9 : 4;
     SeqWork w = {};
-    if (a.seq && c1 - c0 >= SEQ_DIRECT) {
+    *launched += 1;
+    if (a.seq && grav_seq_records(c1 - c0)) {
+        *launched += 6;
         w = seq_work(c1 - c0, a.seq);
         const unsigned nb = (unsigned)((w.lev[0].n + 127) / 128), ng = (unsigned)w.lev[1].n;
         seq_totals_kernel<PASS><<<dim3(nb, NV), 128, 0, s>>>(a, c0, c1, w);
@@ -844,16 +849,17 @@ static cudaError_t seq_run(const GravArgs &a, long long c0, long long c1, double
 }
 
 // A slab's share of the sequential sums: the own planes, continuing acc.
-cudaError_t grav_moments_seq_slab(const GravArgs &a, int pass, double *acc, cudaStream_t s)
+cudaError_t grav_moments_seq_slab(const GravArgs &a, int pass, double *acc, cudaStream_t s, long long *launched)
 {
     const long long sjk = (long long)a.g.ny * a.g.nz;
-    return pass == 0 ? seq_run<0>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s)
-                     : seq_run<1>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s);
+    return pass == 0 ? seq_run<0>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s, launched)
+                     : seq_run<1>(a, a.g.olo * sjk, a.g.ohi * sjk, acc, s, launched);
 }
 
-cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s)
+cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s, long long *launched)
 {
-    if (a.g.n < SEQ_DIRECT) {
+    if (!grav_seq_records(a.g.n)) {
+        *launched += 1;
         seq_direct_kernel<<<1, 288, 0, s>>>(a);
         return cudaGetLastError();
     }
@@ -861,7 +867,9 @@ cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s)
     for (int pass = 0; pass < 2; pass++) {
         cudaError_t e = cudaMemsetAsync(a.scratch, 0, 9 * sizeof(double), s);
         if (e == cudaSuccess)
-            e = pass == 0 ? seq_run<0>(a, 0, a.g.n, a.scratch, s) : seq_run<1>(a, 0, a.g.n, a.scratch, s);
+            e = pass == 0 ? seq_run<0>(a, 0, a.g.n, a.scratch, s, launched)
+                          : seq_run<1>(a, 0, a.g.n, a.scratch, s, launched);
+        *launched += 1;
         if (e == cudaSuccess) e = grav_moments_seq_set(a, pass, a.scratch, s);
         if (e != cudaSuccess) return e;
     }

@@ -179,7 +179,9 @@ struct GravArgs {
 };
 
 // FP64 gravity (bit-exact) -- gravity_fp64.cu
-cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s);
+// (launched: the kernels launched are added to it)
+cudaError_t grav_moments_sequential(const GravArgs &a, cudaStream_t s, long long *launched);
+bool grav_seq_records(long long cells);   // whether sums over so many cells use work memory (GravArgs::seq)
 size_t grav_seq_bytes(const Geom &g);
 cudaError_t grav_moments_tree(const GravArgs &a, cudaStream_t s);
 // Moments of a slab (own planes [a.g.olo, a.g.ohi)).  Sequential order:
@@ -188,7 +190,7 @@ cudaError_t grav_moments_tree(const GravArgs &a, cudaStream_t s);
 // sums (pass 0: M and the centre of mass; pass 1: Q).  Tree order: one
 // partial (9 doubles) per own plane into parts; grav_moments_tree_set adds
 // nparts partials of the whole grid in plane order.
-cudaError_t grav_moments_seq_slab(const GravArgs &a, int pass, double *acc, cudaStream_t s);
+cudaError_t grav_moments_seq_slab(const GravArgs &a, int pass, double *acc, cudaStream_t s, long long *launched);
 cudaError_t grav_moments_seq_set(const GravArgs &a, int pass, const double *acc, cudaStream_t s);
 cudaError_t grav_moments_tree_parts(const GravArgs &a, int pass, double *parts, cudaStream_t s);
 cudaError_t grav_moments_tree_set(const GravArgs &a, int pass, const double *parts, int nparts, cudaStream_t s);
