@@ -288,6 +288,28 @@ static int dmalloc(void **p, size_t bytes)
     return HC_OK;
 }
 
+// For what a call cannot do without.  The buffers that only make solves faster
+// (the records of the moments, the resident sweeps' messages and boundary
+// values) are given back when there is no room beside them.
+static int dmalloc_for(hc_ctx *c, void **p, size_t bytes)
+{
+    if (cudaMalloc(p, bytes) == cudaSuccess) return HC_OK;
+    (void)cudaGetLastError();
+    cudaStreamSynchronize(c->s);
+    cudaFree(c->seq);
+    c->seq = nullptr;
+    if (c->resident == 1) {
+        cudaFree(c->exch);
+        c->exch = nullptr;
+        if (c->cfg.precision == HC_FP64) {
+            cudaFree(c->phi2);
+            c->phi2 = nullptr;
+        }
+        c->resident = -1;
+    }
+    return dmalloc(p, bytes);
+}
+
 static int ensure_res(hc_ctx *c, int max_iter)
 {
     int need = std::max(max_iter, 1) + 16;   // slack for blocked passes
@@ -295,7 +317,7 @@ static int ensure_res(hc_ctx *c, int max_iter)
     cudaFree(c->res);
     c->res = nullptr;
     int cap = std::max(need, 1024);
-    int rc = dmalloc((void **)&c->res, sizeof(double) * cap);
+    int rc = dmalloc_for(c, (void **)&c->res, sizeof(double) * cap);
     if (rc) return rc;
     c->res_cap = cap;
     return HC_OK;
@@ -438,7 +460,7 @@ extern "C" size_t hc_ncells(const hc_ctx *c) { return c ? (size_t)c->g.n : 0; }
 static int ensure_stage(hc_ctx *c)
 {
     if (c->stage) return HC_OK;
-    return dmalloc((void **)&c->stage, 5 * (size_t)c->g.n * sizeof(double));
+    return dmalloc_for(c, (void **)&c->stage, 5 * (size_t)c->g.n * sizeof(double));
 }
 
 static int upload_soa64(hc_ctx *c, const double *q)
@@ -769,13 +791,13 @@ static int sor_fp64(hc_ctx *c, const double *rho)
     double *buf[2] = { c->phi, c->phi2 };
     if (split) {
         const size_t ns = (size_t)split_len(c->g);
-        if (!c->phs) rc = dmalloc((void **)&c->phs, ns * sizeof(double));
-        if (!rc && !c->rhs) rc = dmalloc((void **)&c->rhs, ns * sizeof(double));
+        if (!c->phs) rc = dmalloc_for(c, (void **)&c->phs, ns * sizeof(double));
+        if (!rc && !c->rhs) rc = dmalloc_for(c, (void **)&c->rhs, ns * sizeof(double));
         if (rc) return rc;
     }
     if (wave) {
         if (!c->phi2) {
-            rc = dmalloc((void **)&c->phi2, (size_t)c->g.n * sizeof(double));
+            rc = dmalloc_for(c, (void **)&c->phi2, (size_t)c->g.n * sizeof(double));
             if (rc) return rc;
             buf[1] = c->phi2;
         }
@@ -1217,7 +1239,7 @@ extern "C" int hc_gravity_solve(hc_ctx *c, const double *rho, int with_accel)
     int st;
     if (rho) {
         if (!c->rho_ext) {
-            int rc = dmalloc((void **)&c->rho_ext, n * sizeof(double));
+            int rc = dmalloc_for(c, (void **)&c->rho_ext, n * sizeof(double));
             if (rc) return rc;
         }
         CK(cudaMemcpyAsync(c->rho_ext, rho, n * sizeof(double), cudaMemcpyHostToDevice, c->s));
@@ -1240,9 +1262,9 @@ static int ensure_accel(hc_ctx *c)
 {
     const size_t n = (size_t)c->g.n;
     int rc = HC_OK;
-    if (!c->gx) rc = dmalloc((void **)&c->gx, n * sizeof(double));
-    if (!rc && !c->gy) rc = dmalloc((void **)&c->gy, n * sizeof(double));
-    if (!rc && !c->gz) rc = dmalloc((void **)&c->gz, n * sizeof(double));
+    if (!c->gx) rc = dmalloc_for(c, (void **)&c->gx, n * sizeof(double));
+    if (!rc && !c->gy) rc = dmalloc_for(c, (void **)&c->gy, n * sizeof(double));
+    if (!rc && !c->gz) rc = dmalloc_for(c, (void **)&c->gz, n * sizeof(double));
     return rc;
 }
 
@@ -1402,7 +1424,7 @@ static int step_once(hc_ctx *c, int *grav_status, double *dt_host)
         CK(f64 ? fp64_dt(a, c->s) : fp32_dt(a, c->s));
         t.next(FAM_HYDRO);
         if (f64 && c->cfg.recon == 1) {
-            if (!c->plm && dmalloc((void **)&c->plm, 20 * (size_t)c->g.n * sizeof(double)))
+            if (!c->plm && dmalloc_for(c, (void **)&c->plm, 20 * (size_t)c->g.n * sizeof(double)))
                 return set_err(HC_ERR_NOMEM, "MUSCL-Hancock face-state buffer");
             CK(fp64_plm_interior(a, c->plm, c->s));
             c->launches += 1;
@@ -1492,7 +1514,7 @@ extern "C" int hc_step_host(hc_ctx *c, double *U, double *dt_out)
 // FP64 sums of the current state's 5 conserved fields into sc->cons (no sync).
 static int launch_cons_sums(hc_ctx *c)
 {
-    if (!c->cons_part && dmalloc((void **)&c->cons_part, 5 * (size_t)CONS_BLOCKS * sizeof(double)))
+    if (!c->cons_part && dmalloc_for(c, (void **)&c->cons_part, 5 * (size_t)CONS_BLOCKS * sizeof(double)))
         return set_err(HC_ERR_NOMEM, "conservation-sum partials");
     if (c->cfg.precision == HC_FP64) {
         ConsFields<double> q;
@@ -1722,7 +1744,7 @@ static int slab_buffer(hc_ctx *c, long long need)
     if (c->slab_buf && c->slab_buf_len >= need) return HC_OK;
     cudaFree(c->slab_buf);
     c->slab_buf = nullptr;
-    int rc = dmalloc((void **)&c->slab_buf, (size_t)need * sizeof(double));
+    int rc = dmalloc_for(c, (void **)&c->slab_buf, (size_t)need * sizeof(double));
     if (rc) return rc;
     c->slab_buf_len = need;
     return HC_OK;
@@ -1797,8 +1819,8 @@ extern "C" int hc_slab_sor_begin(hc_ctx *c)
     if (rc) return rc;
     a.res = c->res;
     const size_t ns = (size_t)split_len(c->g);
-    if (!c->phs) rc = dmalloc((void **)&c->phs, ns * sizeof(double));
-    if (!rc && !c->rhs) rc = dmalloc((void **)&c->rhs, ns * sizeof(double));
+    if (!c->phs) rc = dmalloc_for(c, (void **)&c->phs, ns * sizeof(double));
+    if (!rc && !c->rhs) rc = dmalloc_for(c, (void **)&c->rhs, ns * sizeof(double));
     if (rc) return rc;
     if (!c->hslots && cudaMallocHost((void **)&c->hslots, 512 * sizeof(double)) != cudaSuccess)
         return set_err(HC_ERR_NOMEM, "pinned slot buffer");
@@ -2115,7 +2137,7 @@ int ck_buffers(hc_ctx *c, size_t bytes)
         cudaFree(c->ck_dev);
         c->ck_dev = nullptr;
         c->ck_dev_bytes = 0;
-        if (dmalloc((void **)&c->ck_dev, bytes)) return set_err(HC_ERR_NOMEM, "checkpoint packing buffer");
+        if (dmalloc_for(c, (void **)&c->ck_dev, bytes)) return set_err(HC_ERR_NOMEM, "checkpoint packing buffer");
         c->ck_dev_bytes = bytes;
     }
     for (int b = 0; b < 2; b++)
@@ -2314,7 +2336,7 @@ extern "C" int hc_ic_profile_stars(hc_ctx *c, int nstars, const int *n, const do
     }
     CK(cudaSetDevice(c->dev));
     double *tmp = nullptr;
-    if (dmalloc((void **)&tmp, tot * sizeof(double))) return set_err(HC_ERR_NOMEM, "profile tables");
+    if (dmalloc_for(c, (void **)&tmp, tot * sizeof(double))) return set_err(HC_ERR_NOMEM, "profile tables");
     const bool f64 = c->cfg.precision == HC_FP64;
     cudaError_t e = ic_profile_stars(c->g, c->cfg.gamma, nstars, n, r, rho, u, R_star, centre, vel,
                                      f64 ? c->q64[c->cur] : nullptr, f64 ? nullptr : c->q32[c->cur], tmp, c->s);
