@@ -288,6 +288,21 @@ static int dmalloc(void **p, size_t bytes)
     return HC_OK;
 }
 
+// The resident sweeps' messages and, in FP64, boundary values; the context
+// relaxes by the separate sweeps from here on.
+static void drop_resident(hc_ctx *c)
+{
+    if (c->resident == 1) {
+        cudaFree(c->exch);
+        c->exch = nullptr;
+        if (c->cfg.precision == HC_FP64) {
+            cudaFree(c->phi2);
+            c->phi2 = nullptr;
+        }
+    }
+    c->resident = -1;
+}
+
 // For what a call cannot do without.  The buffers that only make solves faster
 // (the records of the moments, the resident sweeps' messages and boundary
 // values) are given back when there is no room beside them.
@@ -298,15 +313,7 @@ static int dmalloc_for(hc_ctx *c, void **p, size_t bytes)
     cudaStreamSynchronize(c->s);
     cudaFree(c->seq);
     c->seq = nullptr;
-    if (c->resident == 1) {
-        cudaFree(c->exch);
-        c->exch = nullptr;
-        if (c->cfg.precision == HC_FP64) {
-            cudaFree(c->phi2);
-            c->phi2 = nullptr;
-        }
-        c->resident = -1;
-    }
+    drop_resident(c);
     return dmalloc(p, bytes);
 }
 
@@ -322,6 +329,9 @@ static int ensure_res(hc_ctx *c, int max_iter)
     c->res_cap = cap;
     return HC_OK;
 }
+
+static void *ensure_seq(hc_ctx *c);
+static bool resident_sweeps(hc_ctx *c, size_t elem);
 
 extern "C" hc_ctx *hc_create(const hc_config *cfg)
 {
@@ -438,6 +448,13 @@ extern "C" hc_ctx *hc_create(const hc_config *cfg)
     if (c->phi) {
         cudaMemsetAsync(c->phi, 0, n * sizeof(double), c->s);
         cudaMemsetAsync(c->phig, 0, n * sizeof(double), c->s);
+    }
+    // what the solves of this configuration run with, where there is room: an
+    // allocation inside the first one stops the whole device for it
+    if (c->gravity) {
+        if (k.precision == HC_FP64 && k.grav_bc == 1 && k.lmax == 0 && k.moment_order == HC_MOMENTS_SEQUENTIAL)
+            ensure_seq(c);
+        resident_sweeps(c, k.precision == HC_FP64 ? sizeof(double) : sizeof(float));
     }
     if (cudaStreamSynchronize(c->s) != cudaSuccess) {
         set_err(HC_ERR_CUDA, "init memset");
@@ -1714,6 +1731,12 @@ extern "C" int hc_set_slab(hc_ctx *c, int gnx, int ioff)
     g.ohi = ohi;
     if (!(c->cfg.dx > 0.0)) g.dx = (c->cfg.xmax - c->cfg.xmin) / gnx;
     c->slab = 1;
+    // a slab's sweeps are separate ones
+    if (c->resident == 1) {
+        CK(cudaSetDevice(c->dev));
+        CK(cudaStreamSynchronize(c->s));
+        drop_resident(c);
+    }
     return HC_OK;
 }
 

@@ -30,3 +30,22 @@ def test_faster_buffers_give_way():
         return phi
 
     assert np.array_equal(solve(True), solve(False))
+
+
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="no CUDA device")
+@pytest.mark.parametrize("precision,later", [(hc.FP32, 0), (hc.FP64, 2 * 128 ** 3 * 8)])
+def test_first_solve_finds_its_buffers(precision, later):
+    """All but the FP64 split fields are there before the first solve."""
+    shape = (128, 128, 128)
+    q = np.zeros((5,) + shape)
+    q[0], q[4] = np.random.default_rng(0).random(shape) + 0.1, 1.0
+
+    def taken():
+        with hc.HydroSolver3D(shape, G=1.0, tol=1e-4, precision=precision) as s:
+            s.set_state(q)
+            before, _ = torch.cuda.mem_get_info()
+            s.gravity_solve()
+            return before - torch.cuda.mem_get_info()[0]
+
+    taken()                                            # loads the kernels
+    assert taken() <= later
