@@ -1063,6 +1063,9 @@ int hc_sor_mixed(hc_ctx *c, const float *rho32)
         // the passes write every interior cell of their output; its boundary
         // cells (zero for the correction) come from here
         if (wave2) CK(cudaMemsetAsync(c->e32b, 0, (size_t)split_len(c->g) * sizeof(float), c->s));
+        // (the streaming passes leave the rows and planes on the grid's faces
+        // alone in both buffers and count on zeros there: hc_create's, and the
+        // network's prediction, which is zero on the faces)
         StreamRun run = { 0, 0 };
         auto pass = [&](int its, int b, int q, int pair, int force) -> int {
             CK(mixed_sor32_stream(a, c->tile[its - 1], its, eb[b], eb[b ^ 1], c->r32, q, pair, thresh, force, c->s));

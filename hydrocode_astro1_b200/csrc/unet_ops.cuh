@@ -352,7 +352,7 @@ __global__ void out_up_kernel(const float *__restrict__ out0, Dims d0, const dou
             if (m >= sp.H) continue;
             const int k0 = 2 * m, k1 = 2 * m + 1;
             const bool in0 = rin && k0 >= 1 && k0 <= sp.nz - 2, in1 = rin && k1 >= 1 && k1 <= sp.nz - 2;
-            float v0 = 0.f, v1 = 0.f;
+            float v0 = 0.f, v1 = 0.f;   // on the grid's faces: the correction sweeps count on zeros there
             if (in0 || in1) {
                 if (in0) {   // lin_coarse(2m): (m-1, m), weight 0.75 on m
                     const float wk = 0.75f;
