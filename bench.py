@@ -322,17 +322,23 @@ def reference_sample(q0, p, sor_iters=10):
 
 # DRAM bytes (read + write) per grid cell of one launch, from ncu captures of
 # the 256^3 workload (profiles/sor_stream_kernel_fp32_stellar_explosion_256.txt,
-# profiles/sor_split_kernel_fp64_stellar_explosion_256.txt), keyed by kernel.
-NCU_DRAM_BYTES_PER_CELL = {"sor_stream_kernel": 12.45, "sor_split_kernel": 14.38}
+# profiles/sor_split_vec_kernel_fp32_stellar_explosion_256.txt,
+# profiles/sor_split_kernel_fp64_stellar_explosion_256.txt), keyed by kernel and word.
+NCU_DRAM_BYTES_PER_CELL = {("sor_stream_kernel", 4): 12.45, ("sor_split_vec_kernel", 4): 6.47,
+                           ("sor_split_kernel", 8): 14.38}
 
 
-def sor_unit(word, iterations, launches):
-    """(kernel, iterations of one unit) of the default relaxation: a launch of
-    thousands of iterations of a grid resident in shared memory (counted per
-    iteration), an FP32 pass of two, an FP64 colour sweep."""
+def sor_unit(word, nz, iterations, launches):
+    """(kernel, iterations of one unit) of the relaxation that ran, by its
+    launches per iteration: a launch of many iterations of a grid resident in
+    shared memory (counted per iteration), an FP32 pass of two, or two colour
+    sweeps (in vectors where the FP32 rows of a colour are whole ones)."""
     if 4 * launches < iterations:
         return "sor_resident_kernel", 1.0
-    return ("sor_stream_kernel", 2.0) if word == 4 else ("sor_split_kernel", 0.5)
+    if word == 4 and 2 * launches < 3 * iterations:
+        return "sor_stream_kernel", 2.0
+    return "sor_split_vec_kernel" if word == 4 and (nz + 1) // 2 % 4 == 0 else "sor_split_kernel", 0.5
+
 
 REF_ITERS_FILE = os.path.join(ROOT, "hydrocode_astro1_b200", "data", "fp64_iterations.json")
 
@@ -429,21 +435,21 @@ def main_ours(args):
 
     # roofline of the dominant kernel, the relaxation's.  Algorithmic bytes of
     # a unit: a pass of two FP32 iterations or one resident iteration 12 B/cell
-    # (e read + write, r read), an FP64 colour sweep half of 24 (phi read +
-    # write, rho read), over the interior cells.  Its time: the SOR family's
+    # (e read + write, r read), a colour sweep half of that, in FP64 of 24 (phi
+    # read + write, rho read), over the interior cells.  Its time: the SOR family's
     # CUDA-event time over the units that counted; it also holds the
     # convergence checks and what was queued past convergence and returns at
     # once, so it is an upper bound.
     interior = (p["shape"][0] - 2) * (p["shape"][1] - 2) * (p["shape"][2] - 2)
     word = 8 if fp64 else 4
-    kname, unit_its = sor_unit(word, sum(r["iters"]), tm["sor_launches"])
+    kname, unit_its = sor_unit(word, p["shape"][2], sum(r["iters"]), tm["sor_launches"])
     bytes_per_launch = interior * 3 * word * min(unit_its, 1.0)
     units = max(sum(r["iters"]) / unit_its, 1)
     sor_avg_ms = tm["sor_ms"] / units
     pk, pk_kind = peaks()
     achieved = bytes_per_launch / (sor_avg_ms / 1e3) / 1e9 if sor_avg_ms > 0 else 0.0
     shares = {k: tm[k] for k in ("hydro_ms", "bc_ms", "sor_ms", "residual_ms", "moments_ms", "unet_ms")}
-    traffic = NCU_DRAM_BYTES_PER_CELL.get(kname)
+    traffic = NCU_DRAM_BYTES_PER_CELL.get((kname, word))
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": pk, "unit": "GB/s",
                 "frac": achieved / pk, "peak_kind": pk_kind,
                 "traffic": traffic * ncell if traffic else None,
