@@ -32,8 +32,8 @@
 // group all CTAs meet, read the norms of its iterations, and either write
 // their block back (the next group's starting point) or, when an iteration
 // inside the group was the last, reload the group's start and run exactly the
-// iterations up to it again.  The first group has four, the next ones at most
-// twice as many as the one before, and where few are left by the norms' rate just
+// iterations up to it again.  The first group has four (an FP32 launch
+// that continues a solve: half of its iterations), the next ones at most twice as many as the one before, and where few are left by the norms' rate just
 // those: a meeting costs half an iteration (64^3) to three (150^3), a group that
 // is too long its iterations twice.  (First groups of 16 made solves of 2 to 14
 // iterations slower than the separate sweeps; a solve of 3 at 64^3 in FP64 took
@@ -71,6 +71,7 @@ struct ResArgs {
     unsigned *meet;            // arrivals (zero at launch)
     double *res;               // update norms by iteration
     int it0, n;                // iterations it0 .. it0 + n - 1
+    int len0;                  // iterations of the first group (FP32)
     double thresh;
     DevScalars *sc;
     unsigned magic;            // ceil(2^32 / vectors per row), 0 for one
@@ -464,7 +465,8 @@ __global__ void __launch_bounds__(RS_NT, 1) sor_resident_kernel(const ResArgs<T>
     if (multi) send_edges(1, ep);
     int t = A.it0;
     const int tend = A.it0 + A.n;
-    int len = multi ? min(4, A.n) : 1;
+    // (FP64 solves hardly ever need a second launch, and their loop has no register to spare)
+    int len = !multi ? 1 : sizeof(T) == 4 ? A.len0 : min(4, A.n);
     int t0 = t, t1 = min(tend, t + len);   // the group of iterations
     int last = -1;                         // the iteration that converged
     bool again = false;                    // the group runs again, up to `last`
@@ -770,6 +772,8 @@ cudaError_t run_resident(const ResPlan &p, T *e, const T *src, const Split &sp, 
     a.res = res;
     a.it0 = it0;
     a.n = n;
+    // a launch that continues a solve has been given the iterations left and a tenth more
+    a.len0 = it0 > 1 ? std::max(4, std::min(n / 2, RS_MAXGROUP)) : 4;
     a.thresh = thresh;
     a.sc = sc;
     a.magic = (unsigned)((0x100000000ULL + (unsigned)(p.Hp / Pack<T>::V) - 1) / (unsigned)(p.Hp / Pack<T>::V));
