@@ -731,7 +731,8 @@ extern "C" int hc_resident_fault(hc_ctx *c, int kind)
 
 // Whether an FP32 context's sweeps run as streaming passes (where they do not
 // run resident).  FP64 keeps the separate sweeps: its windows hold half the
-// cells, and the passes measured 125 us an iteration at 256^3 against 112.
+// cells, and passes of two iterations measured 125 us an iteration at 256^3
+// against 112 (one iteration per pass: not measured).
 static bool stream_sweeps(hc_ctx *c)
 {
     if (c->cfg.sor_depth != 0 || c->cfg.precision != HC_FP32) return false;

@@ -13,7 +13,7 @@
 // rest is 16-byte shared-memory accesses, about four per 16 bytes updated.
 // Microseconds an iteration, separate sweeps -> resident (400 iterations):
 //   FP32  64^3 7.0 -> 5.0   96^3 9.1 -> 5.1   128^3 14.6 -> 8.2   160^3 19.7 -> 12.4   192^3 25.9 -> 15.0
-//   FP64  64^3 6.7 -> 5.5   96^3 12.2 -> 8.0   128^3 16.7 -> 13.1
+//   FP64  64^3 6.7 -> 5.4   96^3 12.2 -> 8.0   128^3 16.7 -> 12.9
 // Small grids are left with the flight of a message (about 1.4 us a half
 // sweep: a store to L2 and a poll of it), large ones with the latency of
 // their 16 warps (the registers' limit; the issue slots are half used).
@@ -22,9 +22,10 @@
 // sweep number}, stored and loaded as one relaxed 64-bit access, so a row
 // needs no fence, no flag line and no second round trip.  A receiver polls
 // the words it needs (bounded; on a timeout the kernel sets sc->lost and
-// leaves, and the caller takes the solve again by the separate sweeps).  One buffer per colour is enough: a sender overwrites its colour's
-// rows two sweeps later, after the receiver's rows of the sweep between,
-// which the receiver sends after it has read the older ones.
+// leaves, and the caller takes the solve again by the separate sweeps).  One
+// buffer per colour is enough: a sender overwrites its colour's rows two
+// sweeps later, after the receiver's rows of the sweep between, which the
+// receiver sends after it has read the older ones.
 //
 // Stop rule.  The solve must end at exactly the first iteration whose update
 // norm is below the threshold, but a grid-wide test per iteration would cost
@@ -32,12 +33,14 @@
 // group all CTAs meet, read the norms of its iterations, and either write
 // their block back (the next group's starting point) or, when an iteration
 // inside the group was the last, reload the group's start and run exactly the
-// iterations up to it again.  The first group has four (an FP32 launch
-// that continues a solve: half of its iterations), the next ones at most twice as many as the one before, and where few are left by the norms' rate just
-// those: a meeting costs half an iteration (64^3) to three (150^3), a group that
-// is too long its iterations twice.  (First groups of 16 made solves of 2 to 14
-// iterations slower than the separate sweeps; a solve of 3 at 64^3 in FP64 took
-// 298 us against 226, now 222; one of 12 350, 266 and 265.)  One CTA alone tests after every iteration.
+// iterations up to it again.  The first group has four (an FP32 launch that
+// continues a solve: half of its iterations), the next ones at most twice as
+// many as the one before, and where few are left by the norms' rate just
+// those: a meeting costs half an iteration (64^3) to three (150^3), a group
+// that is too long its iterations twice.  (First groups of 16 made solves of 2
+// to 14 iterations slower than the separate sweeps.  64^3 FP64, us a solve,
+// sweeps, 16 and now: 3 iterations 226, 298 and 222; 12 iterations 266, 350 and
+// 265.)  One CTA alone tests after every iteration.
 //
 // Per cell the update is SorCoef<T>::update with the operands of the other
 // sweep kernels, and the cells of a colour are independent: the iterates, the

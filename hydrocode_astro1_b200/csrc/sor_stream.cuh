@@ -9,8 +9,10 @@
 // half sweeps.  Microseconds an iteration, separate sweeps -> passes of two:
 //   200^3 28.4 -> 22.0   224^3 35.6 -> 29.6   256^3 47.2 -> 42.3
 //   288^3 103 -> 59.7    320^3 127 -> 71.6    384^3 187 -> 130     512^3 398 -> 287
-// Now bound by latency: 16 warps an SM (the rings take all registers) issue
-// 36% of the time, waiting for loads and shared memory; 2 TB/s of HBM.
+// Now bound by the halo that every window computes again (1.9 updates for one
+// that counts at 256^3, 1.6 at 512^3) and by latency: 16 warps an SM (the rings
+// take all registers) issue 36% of the time, waiting for loads and shared
+// memory; 2 TB/s of HBM at 256^3, 2.8 at 512^3.
 //
 // A CTA owns a tile of rows and vectors (16 bytes, V cells of one colour) of a
 // chunk of planes, plus a halo of NH rows, planes and cells on each side that

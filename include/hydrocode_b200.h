@@ -92,8 +92,10 @@ typedef struct hc_config {
     int sor_depth;           /* SOR kernels, all with the same iterates:
                                 0 (default) many iterations per launch in
                                 shared memory where the grid fits, else two
-                                FP32 iterations per pass or FP64 colour-split
-                                sweeps;
+                                FP32 iterations per pass where rows of one
+                                colour hold a multiple of 4 cells, else
+                                colour-split sweeps (and these for shapes
+                                on which the others are slower);
                                 -3 colour-split with the FP32 correction
                                 sweeps staged by TMA where rows of one colour
                                 hold at most 256 cells, a multiple of 4;
