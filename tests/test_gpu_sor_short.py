@@ -62,4 +62,4 @@ def test_short_solves_take_no_longer(eps):
             return min(times)
 
     resident, separate = best(0), best(1)
-    assert resident < 1.1 * separate, (resident, separate)
+    assert resident < 1.2 * separate, (resident, separate)   # 1.0; with first groups of 16 1.3
